@@ -12,6 +12,7 @@
 #include <atomic>
 #include "plan.h"
 #include "cgemm.cuh"
+#include "diag_lu.cuh"
 #include "factor.h"
 
 namespace aosb {
@@ -67,290 +68,6 @@ __global__ void pad_identity_kernel(int64_t n_pad, const int32_t* __restrict__ p
   if (i >= n_pad || perm[i] >= 0) return;
   const int k = (int)(i / T), r = (int)(i - (int64_t)k * T);
   factor[tile_base(p, n_slots, diag_slot[k], T) + (size_t)r * T + r] = 1.0f;
-}
-
-// ---------------------------------------------------------------------------
-// Diagonal tile: LU with partial pivoting in shared memory + triangle inverses.
-// Rows are padded to T+1 floats so that walking a column touches 32
-// different banks; 512 threads.
-constexpr int kDiagThreads = 512;
-
-template <int T>
-constexpr size_t diag_smem_bytes() {
-  // tile (2 planes, padded rows) + scratch column (2T) + perm (T) + the
-  // recursive-inverse temporaries (2 planes of T*T/2)
-  return (size_t)(2 * T * (T + 1) + 2 * T) * sizeof(float) + T * sizeof(int) +
-         (size_t)T * T * sizeof(float);
-}
-
-template <int T>
-__global__ void __launch_bounds__(kDiagThreads) diag_lu_kernel(int k, const int32_t* __restrict__ diag_slot,
-                                                               int64_t n_slots, int64_t n_pad,
-                                                               float* __restrict__ factor,
-                                                               int32_t* __restrict__ pivots,
-                                                               int32_t* __restrict__ status) {
-  constexpr int LD = T + 1;
-  extern __shared__ float smem[];
-  float* ar = smem;               // T x LD
-  float* ai = smem + T * LD;      // T x LD
-  float* colr = ai + T * LD;      // T  (scratch column)
-  float* coli = colr + T;         // T
-  int* perm = (int*)(coli + T);   // T
-  const int p = blockIdx.x;
-  const int tid = threadIdx.x;
-  float* g = factor + tile_base(p, n_slots, diag_slot[k], T);
-  for (int e = tid; e < T * T; e += kDiagThreads) {
-    const int r = e / T, c = e % T;  // T is a power of two
-    ar[r * LD + c] = g[e];
-    ai[r * LD + c] = g[e + T * T];
-  }
-  for (int r = tid; r < T; r += kDiagThreads) perm[r] = r;
-  __syncthreads();
-  int bad = 0;
-  // Blocked right-looking LU with partial pivoting (LAPACK getrf order):
-  // warp 0 factors each NB-column panel with warp-level syncs only, then all
-  // threads apply the panel's row interchanges to the other columns, form
-  // U12 = inv(L11) A12 and apply the rank-NB update of the trailing block.
-  constexpr int NB = 8;
-  __shared__ int s_swap[NB];
-  const int warp = tid / 32, lane = tid % 32;
-  const int ty = tid / 32, tx = tid % 32;
-  for (int j0 = 0; j0 < T; j0 += NB) {
-    if (warp == 0) {
-      for (int j = j0; j < j0 + NB; ++j) {
-        float best = -1.0f;
-        int bi = j;
-        for (int r = j + lane; r < T; r += 32) {
-          const float m = fabsf(ar[r * LD + j]) + fabsf(ai[r * LD + j]);
-          if (m > best) { best = m; bi = r; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        // every lane now holds the same (best, bi)
-        if (bi != j && lane < NB) {
-          const int c = j0 + lane;
-          float t = ar[j * LD + c]; ar[j * LD + c] = ar[bi * LD + c]; ar[bi * LD + c] = t;
-          t = ai[j * LD + c]; ai[j * LD + c] = ai[bi * LD + c]; ai[bi * LD + c] = t;
-        }
-        if (lane == 0) s_swap[j - j0] = bi;
-        __syncwarp();
-        float pr = ar[j * LD + j], pi = ai[j * LD + j];
-        float d = pr * pr + pi * pi;
-        if (!(d > 0.0f) || !isfinite(d)) {
-          if (lane == 0) bad = isfinite(d) ? kDevZeroPivot : kDevNonFinite;
-          pr = 1.0f; pi = 0.0f; d = 1.0f;
-        }
-        __syncwarp();
-        if (lane == 0) { ar[j * LD + j] = pr; ai[j * LD + j] = pi; }
-        const float ipr = pr / d, ipi = -pi / d;
-        for (int r = j + 1 + lane; r < T; r += 32) {
-          const float xr = ar[r * LD + j], xi = ai[r * LD + j];
-          const float lr = xr * ipr - xi * ipi, li = xr * ipi + xi * ipr;
-          ar[r * LD + j] = lr;
-          ai[r * LD + j] = li;
-          // rank-1 update of the remaining panel columns of row r
-          for (int c = j + 1; c < j0 + NB; ++c) {
-            const float ur = ar[j * LD + c], ui = ai[j * LD + c];
-            ar[r * LD + c] -= lr * ur - li * ui;
-            ai[r * LD + c] -= lr * ui + li * ur;
-          }
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    // row interchanges of this panel, applied in order to the other columns
-    for (int c = tid; c < T; c += kDiagThreads) {
-      if (c >= j0 && c < j0 + NB) continue;
-      for (int t = 0; t < NB; ++t) {
-        const int j = j0 + t, bi = s_swap[t];
-        if (bi != j) {
-          float x = ar[j * LD + c]; ar[j * LD + c] = ar[bi * LD + c]; ar[bi * LD + c] = x;
-          x = ai[j * LD + c]; ai[j * LD + c] = ai[bi * LD + c]; ai[bi * LD + c] = x;
-        }
-      }
-    }
-    if (tid == 0) {
-      for (int t = 0; t < NB; ++t) {
-        const int j = j0 + t, bi = s_swap[t];
-        if (bi != j) { int x = perm[j]; perm[j] = perm[bi]; perm[bi] = x; }
-      }
-    }
-    __syncthreads();
-    // U12 = inv(L11) A12: forward substitution down each column c >= j0+NB
-    for (int c = j0 + NB + tid; c < T; c += kDiagThreads) {
-      for (int j = j0 + 1; j < j0 + NB; ++j) {
-        float sr = ar[j * LD + c], si = ai[j * LD + c];
-        for (int q = j0; q < j; ++q) {
-          const float lr = ar[j * LD + q], li = ai[j * LD + q];
-          const float ur = ar[q * LD + c], ui = ai[q * LD + c];
-          sr -= lr * ur - li * ui;
-          si -= lr * ui + li * ur;
-        }
-        ar[j * LD + c] = sr;
-        ai[j * LD + c] = si;
-      }
-    }
-    __syncthreads();
-    // trailing update A22 -= L21 U12 (rank NB)
-    for (int r = j0 + NB + ty; r < T; r += kDiagThreads / 32) {
-      float lr[NB], li[NB];
-#pragma unroll
-      for (int q = 0; q < NB; ++q) {
-        lr[q] = ar[r * LD + j0 + q];
-        li[q] = ai[r * LD + j0 + q];
-      }
-      for (int c = j0 + NB + tx; c < T; c += 32) {
-        float sr = ar[r * LD + c], si = ai[r * LD + c];
-#pragma unroll
-        for (int q = 0; q < NB; ++q) {
-          const float ur = ar[(j0 + q) * LD + c], ui = ai[(j0 + q) * LD + c];
-          sr -= lr[q] * ur - li[q] * ui;
-          si -= lr[q] * ui + li[q] * ur;
-        }
-        ar[r * LD + c] = sr;
-        ai[r * LD + c] = si;
-      }
-    }
-    __syncthreads();
-  }
-  // Triangle inverses by recursive 2x2 blocking: invert the 8x8 diagonal
-  // blocks (one warp each), then for b = 8, 16, ... , T/2 combine adjacent
-  // blocks:  X12 = -X11 U12 X22  (upper)  and  X21 = -X22 L21 X11  (unit
-  // lower).  tr/ti hold the b x b temporaries of all pairs of a level.
-  float* tr = colr + 2 * T + T;   // after perm (see diag_smem_bytes)
-  float* ti = tr + T * T / 2;
-  // ---- base: 8x8 diagonal blocks, warp w < T/8 takes block w
-  if (warp < T / 8) {
-    const int b0 = warp * 8;
-    const int i = lane % 8;
-    // upper, non-unit: column by column, lane i = row
-    for (int j = 0; j < 8; ++j) {
-      float cr[8], ci[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        cr[q] = ar[(b0 + q) * LD + b0 + j];
-        ci[q] = ai[(b0 + q) * LD + b0 + j];
-      }
-      __syncwarp();
-      const float dd = cr[j] * cr[j] + ci[j] * ci[j];
-      const float dr = cr[j] / dd, di = -ci[j] / dd;
-      if (lane < 8 && i <= j) {
-        if (i == j) {
-          ar[(b0 + j) * LD + b0 + j] = dr;
-          ai[(b0 + j) * LD + b0 + j] = di;
-        } else {
-          float sr = 0.0f, si = 0.0f;
-          for (int q = i; q < j; ++q) {
-            const float xr = ar[(b0 + i) * LD + b0 + q], xi = ai[(b0 + i) * LD + b0 + q];
-            sr += xr * cr[q] - xi * ci[q];
-            si += xr * ci[q] + xi * cr[q];
-          }
-          ar[(b0 + i) * LD + b0 + j] = -(sr * dr - si * di);
-          ai[(b0 + i) * LD + b0 + j] = -(sr * di + si * dr);
-        }
-      }
-      __syncwarp();
-    }
-    // unit lower: columns right to left
-    for (int j = 6; j >= 0; --j) {
-      float cr[8], ci[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        cr[q] = ar[(b0 + q) * LD + b0 + j];
-        ci[q] = ai[(b0 + q) * LD + b0 + j];
-      }
-      __syncwarp();
-      if (lane < 8 && i > j) {
-        float sr = cr[i], si = ci[i];
-        for (int q = j + 1; q < i; ++q) {
-          const float xr = ar[(b0 + i) * LD + b0 + q], xi = ai[(b0 + i) * LD + b0 + q];
-          sr += xr * cr[q] - xi * ci[q];
-          si += xr * ci[q] + xi * cr[q];
-        }
-        ar[(b0 + i) * LD + b0 + j] = -sr;
-        ai[(b0 + i) * LD + b0 + j] = -si;
-      }
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  // ---- combine levels
-  for (int b = 8; b < T; b *= 2) {
-    const int pairs = T / (2 * b);
-    const int per = b * b;
-    // upper: T1 = U12 X22 (X22 upper incl. diagonal)
-    for (int e = tid; e < pairs * per; e += kDiagThreads) {
-      const int m = e / per, r = (e % per) / b, c = e % b;
-      const int A0 = 2 * b * m, B0 = A0 + b;
-      float sr = 0.0f, si = 0.0f;
-      for (int q = 0; q <= c; ++q) {
-        const float ur = ar[(A0 + r) * LD + B0 + q], ui = ai[(A0 + r) * LD + B0 + q];
-        const float xr = ar[(B0 + q) * LD + B0 + c], xi = ai[(B0 + q) * LD + B0 + c];
-        sr += ur * xr - ui * xi;
-        si += ur * xi + ui * xr;
-      }
-      tr[e] = sr;
-      ti[e] = si;
-    }
-    __syncthreads();
-    // X12 = -X11 T1 (X11 upper incl. diagonal), written over U12
-    for (int e = tid; e < pairs * per; e += kDiagThreads) {
-      const int m = e / per, r = (e % per) / b, c = e % b;
-      const int A0 = 2 * b * m, B0 = A0 + b;
-      float sr = 0.0f, si = 0.0f;
-      for (int q = r; q < b; ++q) {
-        const float xr = ar[(A0 + r) * LD + A0 + q], xi = ai[(A0 + r) * LD + A0 + q];
-        const float t_r = tr[m * per + q * b + c], t_i = ti[m * per + q * b + c];
-        sr += xr * t_r - xi * t_i;
-        si += xr * t_i + xi * t_r;
-      }
-      ar[(A0 + r) * LD + B0 + c] = -sr;
-      ai[(A0 + r) * LD + B0 + c] = -si;
-    }
-    __syncthreads();
-    // lower: T1 = L21 X11 (X11 unit lower)
-    for (int e = tid; e < pairs * per; e += kDiagThreads) {
-      const int m = e / per, r = (e % per) / b, c = e % b;
-      const int A0 = 2 * b * m, B0 = A0 + b;
-      float sr = ar[(B0 + r) * LD + A0 + c], si = ai[(B0 + r) * LD + A0 + c];
-      for (int q = c + 1; q < b; ++q) {
-        const float lr = ar[(B0 + r) * LD + A0 + q], li = ai[(B0 + r) * LD + A0 + q];
-        const float xr = ar[(A0 + q) * LD + A0 + c], xi = ai[(A0 + q) * LD + A0 + c];
-        sr += lr * xr - li * xi;
-        si += lr * xi + li * xr;
-      }
-      tr[e] = sr;
-      ti[e] = si;
-    }
-    __syncthreads();
-    // X21 = -X22 T1 (X22 unit lower), written over L21
-    for (int e = tid; e < pairs * per; e += kDiagThreads) {
-      const int m = e / per, r = (e % per) / b, c = e % b;
-      const int A0 = 2 * b * m, B0 = A0 + b;
-      float sr = tr[m * per + r * b + c], si = ti[m * per + r * b + c];
-      for (int q = 0; q < r; ++q) {
-        const float xr = ar[(B0 + r) * LD + B0 + q], xi = ai[(B0 + r) * LD + B0 + q];
-        const float t_r = tr[m * per + q * b + c], t_i = ti[m * per + q * b + c];
-        sr += xr * t_r - xi * t_i;
-        si += xr * t_i + xi * t_r;
-      }
-      ar[(B0 + r) * LD + A0 + c] = -sr;
-      ai[(B0 + r) * LD + A0 + c] = -si;
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < T * T; e += kDiagThreads) {
-    const int r = e / T, c = e % T;
-    g[e] = ar[r * LD + c];
-    g[e + T * T] = ai[r * LD + c];
-  }
-  for (int r = tid; r < T; r += kDiagThreads) pivots[(size_t)p * n_pad + (size_t)k * T + r] = perm[r];
-  if (tid == 0 && bad != 0 && status[p] == 0) status[p] = bad;
 }
 
 // ---------------------------------------------------------------------------
@@ -508,7 +225,7 @@ void step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k) {
   cudaStream_t st = (cudaStream_t)a->stream;
   const int np = a->n_pencils;
   const size_t diag_smem = diag_smem_bytes<T>();
-  diag_lu_kernel<T><<<np, kDiagThreads, diag_smem, st>>>((int)k, P->d_diag_slot, P->n_slots, P->n_pad,
+  diag_lu_kernel<T><<<np, DiagShape<T>::kThreads, diag_smem, st>>>((int)k, P->d_diag_slot, P->n_slots, P->n_pad,
                                                     a->factor, a->pivots, a->status);
   count_launches(1);
   const int nL = P->lb_off[k + 1] - P->lb_off[k];
@@ -580,7 +297,7 @@ int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cu
                      char* err, size_t cap) {
   if (P->T != 128) return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "diagonal step needs tile 128");
   if (int rc = ensure_diag_attr<128>(err, cap)) return rc;
-  diag_lu_kernel<128><<<a->n_pencils, kDiagThreads, diag_smem_bytes<128>(), st>>>(
+  diag_lu_kernel<128><<<a->n_pencils, DiagShape<128>::kThreads, diag_smem_bytes<128>(), st>>>(
       k, P->d_diag_slot, P->n_slots, P->n_pad, a->factor, a->pivots, a->status);
   count_launches(1);
   return 0;
