@@ -28,8 +28,8 @@
 //    row that was a pivot is only retired, and its place is taken when the
 //    block is handed over.
 //
-// The chain that is left is some 200 cycles a pivot (search, broadcast, one
-// update) and the hand-overs; at T = 128 the FP32 pipe in the update is about
+// The chain that is left is 350-450 cycles a pivot (search, broadcast, one
+// update; more beside busy data warps) and the hand-overs; at T = 128 the FP32 pipe in the update is about
 // as long.  The former kernel kept the tile in shared memory (four loads per
 // four FMAs in the inverses) with the panel in line: 283 us at T = 128, 88 us
 // at T = 64 for up to one pencil per SM, against 100 us and 34 us here.

@@ -230,6 +230,8 @@ int plan_upload(aosb_plan* p, char* err, size_t cap) {
       (rc = up(&p->d_ur_tile, p->ur_tile, err, cap)) ||
       (rc = up(&p->d_ua_tile, p->ua_tile, err, cap)) ||
       (rc = up(&p->d_ll_tile, p->ll_tile, err, cap)) ||
+      (rc = up(&p->d_lb_off, p->lb_off, err, cap)) || (rc = up(&p->d_ur_off, p->ur_off, err, cap)) ||
+      (rc = up(&p->d_ua_off, p->ua_off, err, cap)) || (rc = up(&p->d_ll_off, p->ll_off, err, cap)) ||
       (rc = up(&p->d_sc_slot, p->sc_slot, err, cap)) ||
       (rc = up(&p->d_diag_slot, p->diag_slot, err, cap)))
     return rc;
@@ -332,7 +334,8 @@ void build_super_steps(aosb_plan* P) {
 void plan_free_device(aosb_plan* p) {
   int32_t** arrs[] = {&p->d_perm, &p->d_pinv, &p->d_slot, &p->d_lb_slot, &p->d_ur_slot,
                       &p->d_ua_slot, &p->d_ll_slot, &p->d_lb_tile, &p->d_ur_tile,
-                      &p->d_ua_tile, &p->d_ll_tile, &p->d_sc_slot, &p->d_diag_slot,
+                      &p->d_ua_tile, &p->d_ll_tile, &p->d_lb_off, &p->d_ur_off,
+                      &p->d_ua_off, &p->d_ll_off, &p->d_sc_slot, &p->d_diag_slot,
                       &p->d_indices, &p->d_ss_cross, &p->d_ss_rest, &p->d_sp_cross,
                       &p->d_sp_rest};
   for (int32_t** a : arrs) {

@@ -44,6 +44,7 @@ struct aosb_plan {
   int32_t *d_perm = nullptr, *d_pinv = nullptr, *d_slot = nullptr;
   int32_t *d_lb_slot = nullptr, *d_ur_slot = nullptr, *d_ua_slot = nullptr, *d_ll_slot = nullptr;
   int32_t *d_lb_tile = nullptr, *d_ur_tile = nullptr, *d_ua_tile = nullptr, *d_ll_tile = nullptr;
+  int32_t *d_lb_off = nullptr, *d_ur_off = nullptr, *d_ua_off = nullptr, *d_ll_off = nullptr;
   int32_t *d_sc_slot = nullptr, *d_diag_slot = nullptr;
   int32_t *d_ss_cross = nullptr, *d_ss_rest = nullptr;
   int32_t *d_sp_cross = nullptr, *d_sp_rest = nullptr;

@@ -13,6 +13,7 @@
 // Each sweep is right-looking: a diagonal kernel per step, then an update
 // kernel for every off-diagonal tile of that step.
 #include "plan.h"
+#include "solve_cluster.h"
 #include "cgemm.cuh"
 #include "tc_common.cuh"
 #include "timing.h"
@@ -279,6 +280,23 @@ int run_solve(const aosb_plan* P, const aosb_solve_args_v1* a, char* err, size_t
                  (double)np * (2.0 * T * T * sizeof(float) + 2.0 * T * L * sizeof(float2)));
   };
   if (tc) AOSB_CUDA_TRY(cudaMemsetAsync(tc_status, 0, (size_t)np * sizeof(int32_t), st), err, cap);
+  if (tc) {
+    int rc = 0;
+    cudaEvent_t ev[2];
+    const bool timed = timing_begin(st, ev);
+    if (solve_cluster(P, a, tc_status, &rc, err, cap)) {
+      // algorithmic: the update and diagonal work of both sweeps, as below
+      const double tiles = (double)(P->lb_tile.size() + P->ua_tile.size()), diag = 2.0 * P->nb;
+      if (timed)
+        timing_end(kTimedSolveUpdate, st, ev, (8.0 * tiles + 4.0 * diag) * T * T * L * np,
+                   np * (tiles + diag) * (2.0 * T * T * sizeof(float) + 2.0 * T * L * sizeof(float2)));
+      return rc;
+    }
+    if (timed) {
+      cudaEventDestroy(ev[0]);
+      cudaEventDestroy(ev[1]);
+    }
+  }
   int tc_rc = 0;
   // update of step k with the list entries [b, e) of off[k] .. off[k + 1]
   auto update = [&](int k, int64_t b, int64_t e, const int32_t* dtiles, const int32_t* dslots,

@@ -354,6 +354,9 @@ int64_t aosb_tc_set_wait_limit(int64_t polls);
  * updates on the tensor cores in split BF16 (FP32 accumulation); 0 keeps
  * them in FP32 SIMT.  The tensor-core updates bound their waits; after the
  * solves, aosb_solve_check synchronizes the stream and reports a timeout.
+ * Up to some 70 units (pencils x strips of 32 right-hand sides) the sweeps run
+ * as one launch of thread-block clusters, past that as one launch per diagonal
+ * step and one per update; the two forms round differently.
  * ------------------------------------------------------------------------ */
 #define AOSB_SOLVE_TENSOR_CORES 1
 /* AOSB_SOLVE_GRAPH: capture the solve's launch sequence into a CUDA graph
@@ -386,7 +389,8 @@ int aosb_solve(const aosb_plan_t *plan, const aosb_solve_args_v1 *args,
  * aosb_solve). */
 int aosb_solve_check(const aosb_plan_t *plan, const aosb_solve_args_v1 *args,
                      char *err, size_t err_cap);
-/* CTAs per SM of the tensor-core solve update (AOSB_SOLVE_TENSOR_CORES):
+/* CTAs per SM of the tensor-core solve update (AOSB_SOLVE_TENSOR_CORES, the
+ * form with one launch per step):
  * 1 (deep slab and RHS rings, 208 KB of shared memory) or 2 (default:
  * shallow rings, 96 KB each, so one CTA's waits overlap the other's work;
  * bit-identical results); 0 restores the default.  Process-wide; graphs captured before a change
@@ -394,7 +398,8 @@ int aosb_solve_check(const aosb_plan_t *plan, const aosb_solve_args_v1 *args,
  * outside 0..2).  No counterpart in the reference (cuDSS schedules
  * internally). */
 int32_t aosb_solve_set_ctas_per_sm(int32_t ctas);
-/* 1: the tensor-core sweeps (AOSB_SOLVE_TENSOR_CORES) update the next
+/* 1: the tensor-core sweeps (AOSB_SOLVE_TENSOR_CORES, the form with one
+ * launch per step) update the next
  * step's tile first and run the next diagonal solve on a side stream
  * beside the rest of the current step's updates (double-buffered diagonal
  * results; same arithmetic, same results); 0: one diagonal solve and one
