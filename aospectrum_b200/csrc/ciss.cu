@@ -6,6 +6,7 @@
 // norms.  Here they run on the device in FP64 so that the projected
 // problems and the reported residuals carry FP64 accuracy.
 #include "common.cuh"
+#include "dmma.cuh"
 #include "timing.h"
 
 #include <mutex>
@@ -55,53 +56,104 @@ __global__ void moments_kernel(int64_t n, int L, int M, const double2* __restric
 }
 
 // Partial Gram blocks: scratch[chunk][p][q] = sum over rows in chunk of
-// conj(x[j][a]) y[j][b].  grid = (ceil(p/32), ceil(q/32), chunks).
+// conj(x[j][a]) y[j][b].  grid = (ceil(p / TILE), ceil(q / TILE), chunks).
+//
+// FP64 matrix instructions on fragments loaded straight from global memory
+// (the eight columns of a fragment are one 128-byte line of a row; neighbouring
+// warps share lines in L1).  TILE 32: a CTA's four warps own 16 x 16 blocks
+// each over all rows of the chunk.  TILE 16, for grids that would leave SMs
+// idle: the warps split the chunk's rows and add up in shared memory.  The
+// SIMT form it replaces read five shared-memory words per four products: n =
+// 13000, 128 x 128: 436 us, now 66 (floor 46 at 37 TFLOP/s); n = 1715, 96 x
+// 96: 172, now 10.
 constexpr int kGramRows = 512;
 
-__global__ void __launch_bounds__(256) gram_partial_kernel(int64_t n, int p, int q,
+template <int TILE>
+__global__ void __launch_bounds__(128) gram_partial_kernel(int64_t n, int p, int q,
                                                            const double2* __restrict__ x,
                                                            int64_t ldx,
                                                            const double2* __restrict__ y,
                                                            int64_t ldy,
                                                            double2* __restrict__ part) {
-  __shared__ double2 xs[32][33];
-  __shared__ double2 ys[32][33];
-  const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
-  const int64_t r0 = (int64_t)blockIdx.z * kGramRows;
-  const int64_t r1 = (n < r0 + kGramRows) ? n : r0 + kGramRows;
-  const int tid = threadIdx.x;
-  const int ta = tid / 8;          // 32 output rows
-  const int tb = (tid % 8) * 4;    // 4 output columns each
-  double2 acc[4];
+  constexpr bool kSplit = TILE == 16;  // warps split the rows
+  __shared__ double2 sums[kSplit ? 4 : 1][16][17];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int a0 = blockIdx.x * TILE + (kSplit ? 0 : warp / 2 * 16);
+  const int b0 = blockIdx.y * TILE + (kSplit ? 0 : warp % 2 * 16);
+  constexpr int kWarpRows = kSplit ? kGramRows / 4 : kGramRows;
+  const int64_t r0 = (int64_t)blockIdx.z * kGramRows + (kSplit ? warp * kWarpRows : 0);
+  const int64_t r1 = min(n, r0 + kWarpRows);
+  const int col = lane / 4, row = lane % 4;
+  const double2 zero = make_double2(0.0, 0.0);
+  DBlock acc[2][2] = {};
+  const bool va[2] = {a0 + col < p, a0 + 8 + col < p};
+  const bool vb[2] = {b0 + col < q, b0 + 8 + col < q};
+  constexpr int U = 4;  // steps of four rows in flight
+  double2 fa[U][2], fb[U][2];
+  auto load = [&](int u, int64_t r) {
+    const bool in = r + row < r1;
+    const double2* xr = x + (size_t)(r + row) * ldx + a0 + col;
+    const double2* yr = y + (size_t)(r + row) * ldy + b0 + col;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j] = make_double2(0.0, 0.0);
-  for (int64_t r = r0; r < r1; r += 32) {
-    for (int e = tid; e < 32 * 32; e += 256) {
-      const int rr = e / 32, cc = e % 32;
-      const int64_t row = r + rr;
-      xs[rr][cc] = (row < r1 && a0 + cc < p) ? x[(size_t)row * ldx + a0 + cc] : make_double2(0, 0);
-      ys[rr][cc] = (row < r1 && b0 + cc < q) ? y[(size_t)row * ldy + b0 + cc] : make_double2(0, 0);
+    for (int h = 0; h < 2; ++h) {
+      fa[u][h] = in && va[h] ? xr[8 * h] : zero;
+      fb[u][h] = in && vb[h] ? yr[8 * h] : zero;
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int rr = 0; rr < 32; ++rr) {
-      const double2 xv = xs[rr][ta];
+  };
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const double2 yv = ys[rr][tb + j];
-        // conj(xv) * yv
-        acc[j].x = fma(xv.x, yv.x, fma(xv.y, yv.y, acc[j].x));
-        acc[j].y = fma(xv.x, yv.y, fma(-xv.y, yv.x, acc[j].y));
+  for (int u = 0; u < U; ++u) load(u, r0 + 4 * u);
+  for (int64_t r = r0; r < r1; r += 4 * U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 c = make_double2(fa[u][h].x, -fa[u][h].y);  // conj(x)
+        zmma(acc[h][0], c, fb[u][0]);
+        zmma(acc[h][1], c, fb[u][1]);
       }
+      load(u, r + 4 * (U + u));
     }
-    __syncthreads();
   }
-  const int a = a0 + ta;
-  if (a < p) {
-    double2* out = part + (size_t)blockIdx.z * p * q;
+  double2* out = part + (size_t)blockIdx.z * p * q;
+  const int orow = lane / 4, ocol = 2 * (lane % 4);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (b0 + tb + j < q) out[(size_t)a * q + b0 + tb + j] = acc[j];
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int a = 8 * i + orow, b = 8 * j + ocol + e;
+        const double2 v = make_double2(acc[i][j].re[e], acc[i][j].im[e]);
+        if (kSplit)
+          sums[warp][a][b] = v;
+        else if (a0 + a < p && b0 + b < q)
+          out[(size_t)(a0 + a) * q + b0 + b] = v;
+      }
+  if (!kSplit) return;
+  __syncthreads();
+  for (int e = threadIdx.x; e < 256; e += 128) {
+    const int a = e / 16, b = e % 16;
+    if (a0 + a >= p || b0 + b >= q) continue;
+    double2 v = sums[0][a][b];
+#pragma unroll
+    for (int w = 1; w < (kSplit ? 4 : 1); ++w) {
+      v.x += sums[w][a][b].x;
+      v.y += sums[w][a][b].y;
+    }
+    out[(size_t)(a0 + a) * q + b0 + b] = v;
+  }
+}
+
+// TILE 32 needs two CTAs a SM to fill it; below that the finer tiles do.
+void launch_gram_partial(int64_t n, int p, int q, const double2* x, int64_t ldx, const double2* y,
+                         int64_t ldy, double2* part, int chunks, cudaStream_t st) {
+  const int64_t coarse = (int64_t)ceil_div(p, 32) * ceil_div(q, 32) * chunks;
+  if (coarse >= 2 * 148) {
+    dim3 grid(ceil_div(p, 32), ceil_div(q, 32), chunks);
+    gram_partial_kernel<32><<<grid, 128, 0, st>>>(n, p, q, x, ldx, y, ldy, part);
+  } else {
+    dim3 grid(ceil_div(p, 16), ceil_div(q, 16), chunks);
+    gram_partial_kernel<16><<<grid, 128, 0, st>>>(n, p, q, x, ldx, y, ldy, part);
   }
 }
 
@@ -118,86 +170,112 @@ __global__ void gram_reduce_kernel(int chunks, int64_t pq, const double2* __rest
   g[i] = make_double2(sr, si);
 }
 
-// y (n x r) = x (n x p) t (p x r); CTA = 32 rows x 64 columns.
-__global__ void __launch_bounds__(256) dense_mul_kernel(int64_t n, int p, int r,
+// y (n x r) = x (n x p) t (p x r): a warp owns 16 rows x 32 columns, a CTA 64
+// rows, on FP64 matrix instructions with fragments straight from global memory
+// (t stays in L1 and L2).  n = 13000, p = 128, r = 104: 100 us with the former
+// shared-memory form, now 59 (floor 37 at 37 TFLOP/s).
+__global__ void __launch_bounds__(128) dense_mul_kernel(int64_t n, int p, int r,
                                                         const double2* __restrict__ x,
                                                         int64_t ldx,
                                                         const double2* __restrict__ t,
                                                         double2* __restrict__ y, int64_t ldy) {
-  __shared__ double2 xs[32][17];
-  __shared__ double2 ts[16][64];
-  const int64_t r0 = (int64_t)blockIdx.x * 32;
-  const int c0 = blockIdx.y * 64;
-  const int tid = threadIdx.x;
-  const int tr = tid / 16;        // 16 row groups of 2 rows
-  const int tc = tid % 16;        // 16 column groups of 4 columns (strided)
-  double2 acc[2][4];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int64_t r0 = (int64_t)blockIdx.x * 64 + warp * 16;
+  const int c0 = blockIdx.y * 32;
+  if (r0 >= n) return;
+  const int hi = lane / 4, lo = lane % 4;
+  const double2 zero = make_double2(0.0, 0.0);
+  DBlock acc[2][4] = {};
+  const bool vr[2] = {r0 + hi < n, r0 + 8 + hi < n};
+  const double2* xr = x + (size_t)(r0 + hi) * ldx + lo;
+  const double2* tr = t + (size_t)lo * r + c0 + hi;
+  double2 fa[2][2], fb[2][4];
+  auto load = [&](int buf, int k) {
+    const bool in = k + lo < p;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i) fa[buf][i] = in && vr[i] ? xr[(size_t)8 * i * ldx + k] : zero;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0, 0);
-  for (int k0 = 0; k0 < p; k0 += 16) {
-    for (int e = tid; e < 32 * 16; e += 256) {
-      const int rr = e / 16, kk = e % 16;
-      const int64_t row = r0 + rr;
-      xs[rr][kk] = (row < n && k0 + kk < p) ? x[(size_t)row * ldx + k0 + kk] : make_double2(0, 0);
+    for (int j = 0; j < 4; ++j)
+      fb[buf][j] = in && c0 + 8 * j + hi < r ? tr[(size_t)k * r + 8 * j] : zero;
+  };
+  load(0, 0);
+  for (int k = 0; k < p; k += 8) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      load(h ^ 1, k + 4 * (h + 1));
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) zmma(acc[i][j], fa[h][i], fb[h][j]);
     }
-    for (int e = tid; e < 16 * 64; e += 256) {
-      const int kk = e / 64, cc = e % 64;
-      ts[kk][cc] = (k0 + kk < p && c0 + cc < r) ? t[(size_t)(k0 + kk) * r + c0 + cc]
-                                                 : make_double2(0, 0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const double2 a = xs[tr * 2 + i][kk];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double2 b = ts[kk][tc + 16 * j];
-          acc[i][j].x = fma(a.x, b.x, fma(-a.y, b.y, acc[i][j].x));
-          acc[i][j].y = fma(a.x, b.y, fma(a.y, b.x, acc[i][j].y));
-        }
-      }
-    }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const int64_t row = r0 + tr * 2 + i;
-    if (row >= n) continue;
+    if (!vr[i]) continue;
+    double2* out = y + (size_t)(r0 + 8 * i + hi) * ldy + c0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = c0 + tc + 16 * j;
-      if (col < r) y[(size_t)row * ldy + col] = acc[i][j];
-    }
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * j + 2 * lo + e;
+        if (c0 + c < r) out[c] = make_double2(acc[i][j].re[e], acc[i][j].im[e]);
+      }
   }
 }
 
-// out[j] = || a[:, j] - e[j] b[:, j] ||; CTA = 32 columns x 8 row lanes.
-__global__ void column_norms_kernel(int64_t n, int m, const double2* __restrict__ a,
-                                    const double2* __restrict__ b, int64_t ld,
-                                    const double* __restrict__ e, double* __restrict__ out) {
-  __shared__ double part[8][32];
-  const int cl = threadIdx.x % 32, rl = threadIdx.x / 32;
-  const int j = blockIdx.x * 32 + cl;
+// out[j] = || a[:, j] - e[j] b[:, j] ||.  A cluster of kNormCtas CTAs takes
+// eight columns (one 128-byte line of a row) and splits the rows; its first CTA
+// adds the others' sums in rank order from their shared memory, so that the
+// result does not depend on timing and needs no scratch.  One CTA per 32
+// columns, as before, left all but a few SMs idle: n = 13000, 104 columns: 470
+// us, now 35 (floor 7, 43 MB).
+constexpr int kNormCtas = 8, kNormThreads = 256;
+
+__global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads)
+    column_norms_kernel(int64_t n, int m, const double2* __restrict__ a,
+                        const double2* __restrict__ b, int64_t ld, const double* __restrict__ e,
+                        double* __restrict__ out) {
+  __shared__ double part[kNormThreads / 8][9];
+  __shared__ double sum[8];
+  const int rank = (int)blockIdx.x % kNormCtas;
+  const int c = threadIdx.x % 8, rl = threadIdx.x / 8;
+  const int j = (int)(blockIdx.x / kNormCtas) * 8 + c;
   double s = 0.0;
   if (j < m) {
     const double ej = e[j];
-    for (int64_t i = rl; i < n; i += 8) {
+#pragma unroll 4
+    for (int64_t i = (int64_t)rank * (kNormThreads / 8) + rl; i < n;
+         i += kNormCtas * (kNormThreads / 8)) {
       const double2 av = a[(size_t)i * ld + j], bv = b[(size_t)i * ld + j];
       const double dr = av.x - ej * bv.x, di = av.y - ej * bv.y;
       s += dr * dr + di * di;
     }
   }
-  part[rl][cl] = s;
+  part[rl][c] = s;
   __syncthreads();
-  if (rl == 0 && j < m) {
+  if (threadIdx.x < 8) {
     double t = 0.0;
-    for (int q = 0; q < 8; ++q) t += part[q][cl];
+    for (int q = 0; q < kNormThreads / 8; ++q) t += part[q][threadIdx.x];
+    sum[threadIdx.x] = t;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+                   : "memory");
+  if (rank == 0 && threadIdx.x < 8 && j < m) {
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&sum[threadIdx.x]);
+    double t = 0.0;
+    for (int q = 0; q < kNormCtas; ++q) {
+      uint32_t peer;
+      double v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(q));
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(peer) : "memory");
+      t += v;
+    }
     out[j] = sqrt(t);
   }
+  // no CTA leaves while the first may still read its sums
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+                   : "memory");
 }
 
 }  // namespace
@@ -281,9 +359,8 @@ int aosb_gram(int64_t n, int32_t p, int32_t q, const aosb_complex128* x, int64_t
   if (int rc = aosb::gram_grid_check(n, q, err, cap)) return rc;
   const int chunks = (int)((n + aosb::kGramRows - 1) / aosb::kGramRows);
   cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid(aosb::ceil_div(p, 32), aosb::ceil_div(q, 32), chunks);
-  aosb::gram_partial_kernel<<<grid, 256, 0, st>>>(n, p, q, (const double2*)x, ldx,
-                                                  (const double2*)y, ldy, (double2*)scratch);
+  aosb::launch_gram_partial(n, p, q, (const double2*)x, ldx, (const double2*)y, ldy,
+                            (double2*)scratch, chunks, st);
   const int64_t pq = (int64_t)p * q;
   aosb::gram_reduce_kernel<<<aosb::ceil_div(pq, 256), 256, 0, st>>>(
       chunks, pq, (const double2*)scratch, (double2*)g);
@@ -298,8 +375,8 @@ int aosb_dense_mul(int64_t n, int32_t p, int32_t r, const aosb_complex128* x, in
     return aosb::set_error(err, cap, AOSB_ERR_NULL, "null argument");
   if (n <= 0 || p <= 0 || r <= 0 || ldx < p || ldy < r)
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "invalid dense_mul shape");
-  dim3 grid(aosb::ceil_div(n, 32), aosb::ceil_div(r, 64));
-  aosb::dense_mul_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
+  dim3 grid(aosb::ceil_div(n, 64), aosb::ceil_div(r, 32));
+  aosb::dense_mul_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(
       n, p, r, (const double2*)x, ldx, (const double2*)t, (double2*)y, ldy);
   aosb::count_launches(1);
   return aosb::launch_check(err, cap, "dense_mul");
@@ -312,7 +389,8 @@ int aosb_column_norms(int64_t n, int32_t m, const aosb_complex128* a, const aosb
     return aosb::set_error(err, cap, AOSB_ERR_NULL, "null argument");
   if (n <= 0 || m <= 0 || ld < m)
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "invalid norm shape");
-  aosb::column_norms_kernel<<<aosb::ceil_div(m, 32), 256, 0, (cudaStream_t)stream>>>(
+  aosb::column_norms_kernel<<<aosb::kNormCtas * aosb::ceil_div(m, 8), aosb::kNormThreads, 0,
+                              (cudaStream_t)stream>>>(
       n, m, (const double2*)a, (const double2*)b, ld, e, out);
   aosb::count_launches(1);
   return aosb::launch_check(err, cap, "column_norms");
@@ -380,9 +458,8 @@ extern "C" int aosb_gram_noalloc(int64_t n, int32_t p, int32_t q, const aosb_com
   // element that the reduction then reads.
   const int chunks = (int)((n + kGramRows - 1) / kGramRows);
   cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid(ceil_div(p, 32), ceil_div(q, 32), chunks);
-  gram_partial_kernel<<<grid, 256, 0, st>>>(n, p, q, (const double2*)x, ldx, (const double2*)y,
-                                            ldy, (double2*)scratch);
+  launch_gram_partial(n, p, q, (const double2*)x, ldx, (const double2*)y, ldy, (double2*)scratch,
+                      chunks, st);
   const int64_t pq = (int64_t)p * q;
   gram_reduce_kernel<<<ceil_div(pq, 256), 256, 0, st>>>(chunks, pq, (const double2*)scratch,
                                                         (double2*)g);
