@@ -369,11 +369,13 @@ __device__ __forceinline__ void diag_update(float2 (&x)[kDiagBlock][T / 32], int
   }
 }
 
+// `saved`, if given, keeps the real plane of pencil 0's tile as it was found:
+// the Schur complement of everything eliminated before it (tile k at k T^2).
 template <int T>
 __global__ void __launch_bounds__(DiagShape<T>::kThreads, 1)
     diag_lu_kernel(int k, const int32_t* __restrict__ diag_slot, int64_t n_slots, int64_t n_pad,
                    float* __restrict__ factor, int32_t* __restrict__ pivots,
-                   int32_t* __restrict__ status) {
+                   int32_t* __restrict__ status, float* __restrict__ saved) {
   constexpr int NB = kDiagBlock, W = DiagShape<T>::kWarps, CH = DiagShape<T>::kChunks;
   constexpr int kAll = DiagShape<T>::kThreads, kData = W * 32;
   // named barriers, in the order of a block step: block column factored, moved
@@ -417,6 +419,13 @@ __global__ void __launch_bounds__(DiagShape<T>::kThreads, 1)
       const int e = (row0 + r) * T + lane + 32 * j;
       x[r][j] = make_float2(g[e], g[e + T * T]);
     }
+  if (saved != nullptr && p == 0) {
+#pragma unroll
+    for (int r = 0; r < NB; ++r)
+#pragma unroll
+      for (int j = 0; j < CH; ++j)
+        saved[(size_t)k * (T * T) + (row0 + r) * T + lane + 32 * j] = x[r][j].x;
+  }
   for (int b = 0; b < W; ++b) {
     const int k0 = b * NB, next = k0 + NB;
     diag_bar_sync(kBarFactored, kAll);

@@ -221,12 +221,13 @@ int ensure_diag_attr(char* err, size_t cap) {
 
 // Diagonal LU and panel updates of step k (FP32 SIMT).
 template <int T>
-void step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k) {
+void step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k,
+                 float* diag_tiles = nullptr) {
   cudaStream_t st = (cudaStream_t)a->stream;
   const int np = a->n_pencils;
   const size_t diag_smem = diag_smem_bytes<T>();
   diag_lu_kernel<T><<<np, DiagShape<T>::kThreads, diag_smem, st>>>((int)k, P->d_diag_slot, P->n_slots, P->n_pad,
-                                                    a->factor, a->pivots, a->status);
+                                                    a->factor, a->pivots, a->status, diag_tiles);
   count_launches(1);
   const int nL = P->lb_off[k + 1] - P->lb_off[k];
   const int nU = P->ur_off[k + 1] - P->ur_off[k];
@@ -241,14 +242,12 @@ void step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k) {
 
 template <int T>
 int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
-              StepHook hook, void* hook_ctx) {
+              float* diag_tiles) {
   cudaStream_t st = (cudaStream_t)a->stream;
   const int np = a->n_pencils;
   if (int rc = ensure_diag_attr<T>(err, cap)) return rc;
   for (int64_t k = 0; k < P->nb; ++k) {
-    if (hook != nullptr)
-      if (int rc = hook(hook_ctx, k, st, err, cap)) return rc;
-    step_panels<T>(P, a, k);
+    step_panels<T>(P, a, k, diag_tiles);
     const int nL = P->lb_off[k + 1] - P->lb_off[k];
     const int nU = P->ur_off[k + 1] - P->ur_off[k];
     if (nL > 0 && nU > 0) {
@@ -298,17 +297,17 @@ int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cu
   if (P->T != 128) return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "diagonal step needs tile 128");
   if (int rc = ensure_diag_attr<128>(err, cap)) return rc;
   diag_lu_kernel<128><<<a->n_pencils, DiagShape<128>::kThreads, diag_smem_bytes<128>(), st>>>(
-      k, P->d_diag_slot, P->n_slots, P->n_pad, a->factor, a->pivots, a->status);
+      k, P->d_diag_slot, P->n_slots, P->n_pad, a->factor, a->pivots, a->status, nullptr);
   count_launches(1);
   return 0;
 }
 
 int factor_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
-                 StepHook hook, void* hook_ctx) {
+                 float* diag_tiles) {
   switch (P->T) {
-    case 32: return run_plain<32>(P, a, err, cap, hook, hook_ctx);
-    case 64: return run_plain<64>(P, a, err, cap, hook, hook_ctx);
-    case 128: return run_plain<128>(P, a, err, cap, hook, hook_ctx);
+    case 32: return run_plain<32>(P, a, err, cap, diag_tiles);
+    case 64: return run_plain<64>(P, a, err, cap, diag_tiles);
+    case 128: return run_plain<128>(P, a, err, cap, diag_tiles);
   }
   return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "unsupported tile size");
 }

@@ -11,12 +11,11 @@ int factor_step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int k, 
                        size_t cap);
 int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cudaStream_t st,
                      char* err, size_t cap);
-// Called by the plain factorization before the diagonal LU of tile step k,
-// on the factorization's stream: the diagonal tile (k, k) then holds the
-// Schur complement that the steps before k left (nonzero return aborts).
-using StepHook = int (*)(void* ctx, int64_t k, cudaStream_t stream, char* err, size_t cap);
+// `diag_tiles`, if given (T^2 floats per tile step): the real plane of pencil
+// 0's diagonal tile of each step as its LU found it, that is, the Schur
+// complement that the steps before left.
 int factor_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
-                 StepHook hook = nullptr, void* hook_ctx = nullptr);
+                 float* diag_tiles = nullptr);
 int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap);
 size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils);
 // Two-CTA (M = 256) Schur update of one pair list (schur_pair.cu): the

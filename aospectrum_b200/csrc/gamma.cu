@@ -21,10 +21,13 @@
 // (Haynsworth), In(A) = In(A_11) + In(A / A_11), applied tile by tile,
 // In(A) = sum_k In(S_kk), and by Sylvester's law In(A) counts the
 // eigenvalues of the pencil (H, S) (S positive definite) below, at and
-// above sigma.  A hook on the factorization stream runs, before each
-// diagonal LU, a Bunch-Kaufman symmetric-indefinite LDL^T of S_kk in FP64
-// shared memory (1x1 and 2x2 pivots, alpha = (1 + sqrt(17)) / 8) and adds
-// the signs of its D blocks to the counters.  Padding rows of the plan are
+// above sigma.  The diagonal LU of every step keeps the S_kk it found, and
+// after the factorization one launch with a CTA per tile runs a Bunch-Kaufman
+// symmetric-indefinite LDL^T of each in FP64 shared memory (1x1 and 2x2
+// pivots, alpha = (1 + sqrt(17)) / 8) and adds the signs of its D blocks to the
+// counters.  (Run between the steps, one CTA at a time, those LDL^Ts were
+// nearly half of a factorization: n = 4459, 70 tiles of 64: 11.0 of 24.4 ms,
+// now 0.2.)  Padding rows of the plan are
 // identity rows: each adds one positive count, removed on the host.
 #include "plan.h"
 #include "factor.h"
@@ -80,22 +83,20 @@ __device__ __forceinline__ void block_argmax(double v, int idx, double* s_val, i
   __syncthreads();
 }
 
-// Inertia of the symmetric diagonal tile (k, k) of pencil blockIdx.x by a
-// Bunch-Kaufman LDL^T (partial pivoting) in FP64 shared memory; adds
-// (negative, zero, positive) counts and the number of symmetric
-// interchanges to counts[p][0..3].  The real plane of the tile is read; it
+// Inertia of the symmetric tile blockIdx.x of `tiles` by a Bunch-Kaufman LDL^T
+// (partial pivoting) in FP64 shared memory; adds (negative, zero, positive)
+// counts and the number of symmetric interchanges to counts[0..3].  The tile
 // is symmetrized as (A + A^T) / 2 against FP32 rounding of the updates.
 template <int T>
 __global__ void __launch_bounds__(kInertiaThreads) tile_inertia_kernel(
-    int k, const int32_t* __restrict__ diag_slot, int64_t n_slots,
-    const float* __restrict__ factor, int32_t* __restrict__ counts) {
+    const float* __restrict__ tiles, int32_t* __restrict__ counts) {
   constexpr int LD = T + 1;
   extern __shared__ double a[];
   __shared__ double s_val[kInertiaThreads / 32];
   __shared__ int s_idx[kInertiaThreads / 32];
-  __shared__ int s_step, s_kind, s_swap_from, s_swap_to;
-  const int p = blockIdx.x, tid = threadIdx.x;
-  const float* g = factor + ((size_t)p * n_slots + diag_slot[k]) * (size_t)(2 * T * T);
+  __shared__ int s_kind, s_swap_from, s_swap_to;
+  const int tid = threadIdx.x;
+  const float* g = tiles + (size_t)blockIdx.x * (T * T);
   for (int e = tid; e < T * T; e += kInertiaThreads) {
     const int r = e / T, c = e % T;
     a[r * LD + c] = 0.5 * ((double)g[r * T + c] + (double)g[c * T + r]);
@@ -208,12 +209,11 @@ __global__ void __launch_bounds__(kInertiaThreads) tile_inertia_kernel(
     }
   }
   if (tid == 0) {
-    atomicAdd(&counts[4 * p + 0], neg);
-    atomicAdd(&counts[4 * p + 1], zero);
-    atomicAdd(&counts[4 * p + 2], pos);
-    atomicAdd(&counts[4 * p + 3], swaps);
+    atomicAdd(&counts[0], neg);
+    atomicAdd(&counts[1], zero);
+    atomicAdd(&counts[2], pos);
+    atomicAdd(&counts[3], swaps);
   }
-  (void)s_step;
 }
 
 // Symmetric-pattern values from the caller's real CSR values: entry q of
@@ -269,6 +269,7 @@ struct aosb_shift_factor {
   int32_t* d_pk = nullptr;
   double2* d_shift = nullptr;
   int32_t* d_counts = nullptr;
+  float* d_tiles = nullptr;  // diagonal tiles as their LU found them
   float2* d_work = nullptr;
   void* d_scratch = nullptr;
   aosb_shift_factor_stats stats{};
@@ -277,27 +278,22 @@ struct aosb_shift_factor {
 namespace aosb {
 namespace {
 
-int inertia_hook(void* ctx, int64_t k, cudaStream_t st, char* err, size_t cap) {
-  aosb_shift_factor* f = (aosb_shift_factor*)ctx;
-  const aosb_plan* P = f->plan;
-  switch (P->T) {
-    case 32:
-      tile_inertia_kernel<32><<<1, kInertiaThreads, inertia_smem_bytes<32>(), st>>>(
-          (int)k, P->d_diag_slot, P->n_slots, f->d_factor, f->d_counts);
-      break;
-    case 64:
-      tile_inertia_kernel<64><<<1, kInertiaThreads, inertia_smem_bytes<64>(), st>>>(
-          (int)k, P->d_diag_slot, P->n_slots, f->d_factor, f->d_counts);
-      break;
-    case 128:
-      tile_inertia_kernel<128><<<1, kInertiaThreads, inertia_smem_bytes<128>(), st>>>(
-          (int)k, P->d_diag_slot, P->n_slots, f->d_factor, f->d_counts);
-      break;
-    default:
-      return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "unsupported tile size");
+template <int T>
+void launch_inertia(const aosb_shift_factor* f) {
+  tile_inertia_kernel<T><<<(unsigned)f->plan->nb, kInertiaThreads, inertia_smem_bytes<T>(),
+                           f->stream>>>(f->d_tiles, f->d_counts);
+}
+
+// Adds up the inertia of the tiles that the factorization kept.
+int tile_inertias(const aosb_shift_factor* f, char* err, size_t cap) {
+  switch (f->plan->T) {
+    case 32: launch_inertia<32>(f); break;
+    case 64: launch_inertia<64>(f); break;
+    case 128: launch_inertia<128>(f); break;
+    default: return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "unsupported tile size");
   }
   count_launches(1);
-  return 0;
+  return launch_check(err, cap, "tile inertia");
 }
 
 int inertia_attributes(int T, char* err, size_t cap) {
@@ -338,7 +334,8 @@ int factorize(aosb_shift_factor* f, float shift, char* err, size_t cap) {
                          f->d_factor, f->d_piv, f->d_status, nullptr, f->stream};
   if (int rc = inertia_attributes((int)P->T, err, cap)) return rc;
   if (int rc = factor_assemble(P, &fa, err, cap)) return rc;
-  if (int rc = factor_plain(P, &fa, err, cap, inertia_hook, f)) return rc;
+  if (int rc = factor_plain(P, &fa, err, cap, f->d_tiles)) return rc;
+  if (int rc = tile_inertias(f, err, cap)) return rc;
   int32_t counts[4] = {0, 0, 0, 0}, status = 0;
   AOSB_CUDA_TRY(cudaMemcpyAsync(counts, f->d_counts, sizeof(counts), cudaMemcpyDeviceToHost,
                                 f->stream), err, cap);
@@ -385,6 +382,7 @@ void aosb_shift_factor_destroy(aosb_shift_factor_t* f) {
   cudaFree(f->d_pk);
   cudaFree(f->d_shift);
   cudaFree(f->d_counts);
+  cudaFree(f->d_tiles);
   cudaFree(f->d_work);
   cudaFree(f->d_scratch);
   if (f->plan) aosb_plan_destroy(f->plan);
@@ -488,6 +486,7 @@ int aosb_shift_factor_create_device(aosb_shift_factor_t** out, int64_t n, int64_
   };
   const size_t fbytes = aosb_factor_bytes(P, 1);
   const size_t scratch = aosb_solve_scratch_bytes(P, 1, maximum_rhs);
+  const size_t tile_bytes = sizeof(float) * (size_t)(P->nb * P->T * P->T);
   const int32_t zero = 0;
   if ((rc = alloc((void**)&f->d_src, sizeof(int32_t) * nsym, "source positions")) ||
       (rc = alloc((void**)&f->d_h, sizeof(float2) * nsym, "H values")) ||
@@ -498,6 +497,7 @@ int aosb_shift_factor_create_device(aosb_shift_factor_t** out, int64_t n, int64_
       (rc = alloc((void**)&f->d_pk, sizeof(int32_t), "pencil index")) ||
       (rc = alloc((void**)&f->d_shift, sizeof(double2), "shift")) ||
       (rc = alloc((void**)&f->d_counts, 4 * sizeof(int32_t), "inertia counters")) ||
+      (rc = alloc((void**)&f->d_tiles, tile_bytes, "diagonal tiles")) ||
       (rc = alloc((void**)&f->d_work, sizeof(float2) * P->n_pad * maximum_rhs, "solve block")) ||
       (rc = alloc(&f->d_scratch, scratch > 16 ? scratch : 16, "solve scratch"))) {
     aosb_shift_factor_destroy(f);
@@ -512,7 +512,7 @@ int aosb_shift_factor_create_device(aosb_shift_factor_t** out, int64_t n, int64_
     aosb_shift_factor_destroy(f);
     return set_error(err, cap, AOSB_ERR_CUDA, "shift-factor upload failed: %s", cudaGetErrorString(e));
   }
-  f->stats.permanent_device_bytes = fbytes + sizeof(int32_t) * P->n_pad +
+  f->stats.permanent_device_bytes = fbytes + tile_bytes + sizeof(int32_t) * P->n_pad +
                                     (sizeof(int32_t) + 2 * sizeof(float2)) * nsym;
   f->stats.peak_device_bytes = f->stats.permanent_device_bytes +
                                sizeof(float2) * P->n_pad * maximum_rhs + scratch;
