@@ -8,11 +8,11 @@
 // CSR arrays, because every row of atom i has the same column structure.
 // Entry (a, c) of group (i, j) sits at dst_base + a * rowlen_i + c.
 //
-// The device kernel gives one warp to each group (window) and chunk of up
-// to four k points: it sums the member blocks of (i, j) and of its mirror
-// (j, i) in block order (the order the reference's stable sort leaves them
-// in), applies the Hermitian projection of sparse.py:25-36 and writes the
-// window row by row for every k point of the chunk.  With
+// The device kernel gives a CTA a strip of up to eight neighbouring windows of
+// one row atom and all k points (in chunks of four): it sums the member blocks
+// of (i, j) and of its mirror (j, i) in block order (the order the reference's
+// stable sort leaves them in), applies the Hermitian projection of
+// sparse.py:25-36 and writes the strip row by row.  With
 // real block values the products v * phase are exact, so the output is
 // bit-identical to the reference's numpy path.
 #include "common.cuh"
@@ -37,12 +37,14 @@ struct aosb_bloch {
   int2* d_group_members = nullptr; // [begin, end) into members
   int64_t* d_member_off = nullptr; // value offset of each member block
   int32_t* d_member_shift = nullptr;
+  int2* d_strips = nullptr;        // [first, last) groups of each strip
   // host copies of the device tables (uploaded by aosb_bloch_upload)
   std::vector<int4> g_info;
   std::vector<int64_t> g_dst;
   std::vector<int2> g_mem;
   std::vector<int64_t> m_off;
   std::vector<int32_t> m_shift;
+  std::vector<int2> strips;
   int64_t n_values = 0;  // stored block values (sum of block sizes), set at upload
   bool uploaded = false;
 };
@@ -83,8 +85,7 @@ __device__ __forceinline__ float2 cmul_rn(float2 a, float2 b) {
                      __fadd_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x)));
 }
 
-// k points per warp: one warp reads its blocks once and writes this many
-// H(k), S(k) windows (four keeps the kernel at 64 registers, 32 warps per SM)
+// k points whose phases a thread holds at a time
 constexpr int kBlochKChunk = 4;
 
 // Sums of one element over the member blocks [range.x, range.y) of a group
@@ -120,128 +121,187 @@ __device__ __forceinline__ float2 hermitian_mean(float2 x, float2 y) {
   return make_float2(__fmul_rn(__fadd_rn(x.x, y.x), 0.5f), __fmul_rn(__fsub_rn(x.y, y.y), 0.5f));
 }
 
-// One warp per group (i, j) writes that group's window.  Groups are sorted by
-// (row atom, column atom), so the 8 warps of a CTA write neighbouring windows
-// of the same CSR rows at the same time and the 32-byte sectors they share
-// at window boundaries are completed in L2 instead of leaving it partly
-// written.  Element (a, c) of window (i, j) and element (c, a) of its mirror
-// (j, i) hold the Hermitian mean of the pair and its conjugate: the upper
-// window (i < j) writes mean(x_ij(a, c), x_ji(c, a)), the lower window writes
-// the conjugate of its upper mirror's mean formed the same way.
+// Strips: neighbouring windows (i, j) of one row atom, whose segments of each
+// CSR row are contiguous; at most kStripWindows of them, kStripColumns columns
+// and kStripValues elements (a longer window is a strip of its own).
+constexpr int kStripWindows = 8, kStripColumns = 128, kStripValues = 1376;
+constexpr int kStripThreads = 256;
+
+// Element (a, c) of window (i, j) and element (c, a) of its mirror (j, i) hold
+// the Hermitian mean of the pair and its conjugate: the upper window (i < j)
+// writes mean(x_ij(a, c), x_ji(c, a)), the lower window writes the conjugate of
+// its upper mirror's mean formed the same way; in a diagonal window the
+// elements above and below the diagonal do so, and the diagonal keeps its real
+// part.
+
+// One warp, one window, any number of member blocks.
 template <typename V>
-__global__ void __launch_bounds__(256, 4) bloch_windows_kernel(
-    int64_t n_groups, const int4* __restrict__ group, const int64_t* __restrict__ gdst,
-    const int2* __restrict__ gmem, const int64_t* __restrict__ moff,
-    const int32_t* __restrict__ msh, const V* __restrict__ hv, const V* __restrict__ sv,
-    const float2* __restrict__ phases, int64_t n_shifts, int64_t nnz, int n_k,
-    float2* __restrict__ hout, float2* __restrict__ sout) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (warp >= n_groups) return;
-  const int k0 = blockIdx.y * kBlochKChunk;
-  const int nk = min(n_k - k0, kBlochKChunk);
+__device__ __forceinline__ void window_sums(int g, int lane, int k0, int nk,
+                                            const int4* __restrict__ group,
+                                            const int64_t* __restrict__ gdst,
+                                            const int2* __restrict__ gmem,
+                                            const int64_t* __restrict__ moff,
+                                            const int32_t* __restrict__ msh,
+                                            const V* __restrict__ hv, const V* __restrict__ sv,
+                                            const float2* __restrict__ phases, int64_t n_shifts,
+                                            int64_t nnz, float2* __restrict__ hout,
+                                            float2* __restrict__ sout) {
   const float2* ph0 = phases + (int64_t)k0 * n_shifts;
-  const int64_t out0 = (int64_t)k0 * nnz;
-  const int g = (int)warp;
   const int4 gi = group[g];  // nr, nc, rowlen, mirror
   const int nr = gi.x, nc = gi.y, rl = gi.z, gm = gi.w;
   const int ne = nr * nc;
-  const int64_t base = gdst[g];
-  const int2 rg = gmem[g];
+  const int64_t at0 = (int64_t)k0 * nnz + gdst[g];
+  const int2 rg = gmem[g], mr = gmem[gm];
   float2 x[kBlochKChunk], y[kBlochKChunk];
-  if (gm == g) {
-    // diagonal window: t runs over [matrix H|S][row-major element]; the mean
-    // of the pair (lo, hi) is formed the same way for both of its entries
-    for (int t = lane; t < 2 * ne; t += 32) {
-      const int which = t >= ne;
-      const int e = t - which * ne;
-      const int a = e / nc, c = e - (e / nc) * nc;
-      const V* vals = which == 0 ? hv : sv;
-      float2* out = (which == 0 ? hout : sout) + out0 + base + (int64_t)a * rl + c;
-      const int lo = min(a, c), hi = max(a, c);
-      group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, rg, lo * nc + hi, x);
-      if (a != c) group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, rg, hi * nc + lo, y);
-#pragma unroll
-      for (int q = 0; q < kBlochKChunk; ++q) {
-        if (q < nk) {
-          float2 v;
-          if (a == c) {
-            v = make_float2(x[q].x, 0.0f);
-          } else {
-            const float2 mean = hermitian_mean(x[q], y[q]);
-            v = a < c ? mean : make_float2(mean.x, -mean.y);
-          }
-          out[q * nnz] = v;
-        }
-      }
-    }
-    return;
-  }
-  const bool lower = gm < g;
-  const int2 mr = gmem[gm];
-  // the mean's first operand comes from the upper group of the pair
-  const int2 r1 = lower ? mr : rg, r2 = lower ? rg : mr;
-  if (r1.y - r1.x == 1 && r2.y - r2.x == 1) {
-    // One member block each way (a single lattice image, the common case):
-    // value offsets and phases are warp-uniform and loaded once; each lane
-    // keeps two elements' value loads in flight.
-    const int64_t o1 = moff[r1.x], o2 = moff[r2.x];
-    const float2* ph1 = ph0 + msh[r1.x];
-    const float2* ph2 = ph0 + msh[r2.x];
-    float2 p1[kBlochKChunk], p2[kBlochKChunk];
-#pragma unroll
-    for (int q = 0; q < kBlochKChunk; ++q) {
-      p1[q] = q < nk ? ph1[q * n_shifts] : make_float2(0.0f, 0.0f);
-      p2[q] = q < nk ? ph2[q * n_shifts] : make_float2(0.0f, 0.0f);
-    }
-    for (int t0 = lane; t0 < 2 * ne; t0 += 64) {
-      float2 v1[2], v2[2];
-      float2* out[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int t = t0 + 32 * u;
-        out[u] = nullptr;
-        v1[u] = v2[u] = make_float2(0.0f, 0.0f);
-        if (t < 2 * ne) {
-          const int which = t >= ne;
-          const int e = t - which * ne;
-          const int a = e / nc, c = e - a * nc;
-          const int eg = a * nc + c, em = c * nr + a;
-          const V* vals = which == 0 ? hv : sv;
-          out[u] = (which == 0 ? hout : sout) + out0 + base + (int64_t)a * rl + c;
-          v1[u] = load_value<V>(vals, o1 + (lower ? em : eg));
-          v2[u] = load_value<V>(vals, o2 + (lower ? eg : em));
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (out[u] == nullptr) continue;
-#pragma unroll
-        for (int q = 0; q < kBlochKChunk; ++q) {
-          if (q < nk) {
-            const float2 mean = hermitian_mean(cmul_rn(v1[u], p1[q]), cmul_rn(v2[u], p2[q]));
-            out[u][q * nnz] = lower ? make_float2(mean.x, -mean.y) : mean;
-          }
-        }
-      }
-    }
-    return;
-  }
-  // general: t runs over [matrix H|S][row-major element]
+  // t runs over [matrix H|S][row-major element]
   for (int t = lane; t < 2 * ne; t += 32) {
     const int which = t >= ne;
     const int e = t - which * ne;
     const int a = e / nc, c = e - a * nc;
     const int eg = a * nc + c, em = c * nr + a;
+    const bool lower = gm < g || (gm == g && a > c);
     const V* vals = which == 0 ? hv : sv;
-    float2* out = (which == 0 ? hout : sout) + out0 + base + (int64_t)a * rl + c;
-    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, r1, lower ? em : eg, x);
-    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, r2, lower ? eg : em, y);
+    float2* out = (which == 0 ? hout : sout) + at0 + (int64_t)a * rl + c;
+    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, lower ? mr : rg, lower ? em : eg, x);
+    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, lower ? rg : mr, lower ? eg : em, y);
 #pragma unroll
     for (int q = 0; q < kBlochKChunk; ++q) {
       if (q < nk) {
         const float2 mean = hermitian_mean(x[q], y[q]);
-        out[q * nnz] = lower ? make_float2(mean.x, -mean.y) : mean;
+        float2 v = lower ? make_float2(mean.x, -mean.y) : mean;
+        if (gm == g && a == c) v = make_float2(x[q].x, 0.0f);
+        out[q * nnz] = v;
+      }
+    }
+  }
+}
+
+// One CTA per strip (x) and share of the k chunks (y).  Where every window of
+// the strip has one member block each way (a single lattice image, the common
+// case) the blocks are copied to shared memory, contiguous as they are stored,
+// with all copies in flight at once; then a thread keeps one column of the
+// strip, its window's phases in registers, and walks the rows: a warp writes
+// 256 contiguous bytes of a CSR row.  A warp per window, as before, gathered
+// single values in rounds of two per lane and was bound by their latency (43 %
+// of the copy bandwidth).  4096 atoms, 13 orbitals, 4 k points (4.6 GB): 1.60
+// ms, now 1.08 (0.70 at the copy bandwidth; streaming stores and other register
+// limits were slower); 64 atoms, 1 k point: 9.8 us, now 5.8.
+template <typename V>
+__global__ void __launch_bounds__(kStripThreads) bloch_strips_kernel(
+    const int2* __restrict__ strips, const int4* __restrict__ group,
+    const int64_t* __restrict__ gdst, const int2* __restrict__ gmem,
+    const int64_t* __restrict__ moff, const int32_t* __restrict__ msh, const V* __restrict__ hv,
+    const V* __restrict__ sv, const float2* __restrict__ phases, int64_t n_shifts, int64_t nnz,
+    int n_k, float2* __restrict__ hout, float2* __restrict__ sout) {
+  // [own, mirror block][H, S][values of the strip's windows in turn]
+  __shared__ V vals[2][2][kStripValues];
+  __shared__ int first_value[kStripWindows], first_column[kStripWindows + 1], widths[kStripWindows];
+  __shared__ int mirrors[kStripWindows], own_shift[kStripWindows], mirror_shift[kStripWindows];
+  __shared__ int fast;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int2 st = strips[blockIdx.x];
+  const int nw = st.y - st.x;
+  const int chunks = (n_k + kBlochKChunk - 1) / kBlochKChunk;
+  if (warp == 0) {
+    // window tables: one lane per window, prefix sums by shuffles
+    int4 gi = make_int4(0, 0, 0, 0);
+    int2 rg = make_int2(0, 0), mr = make_int2(0, 0);
+    if (lane < nw) {
+      gi = group[st.x + lane];
+      rg = gmem[st.x + lane];
+      mr = gmem[gi.w];
+    }
+    int cols = gi.y, values = gi.x * gi.y;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int c = __shfl_up_sync(0xffffffffu, cols, o), v = __shfl_up_sync(0xffffffffu, values, o);
+      if (lane >= o) {
+        cols += c;
+        values += v;
+      }
+    }
+    const bool single = lane >= nw || (rg.y - rg.x == 1 && mr.y - mr.x == 1);
+    const bool all = __all_sync(0xffffffffu, single ? 1 : 0) != 0;
+    const int width = __shfl_sync(0xffffffffu, cols, 31), total = __shfl_sync(0xffffffffu, values, 31);
+    const bool ok = all && width <= kStripColumns && total <= kStripValues;
+    if (lane < nw) {
+      first_column[lane] = cols - gi.y;
+      first_value[lane] = values - gi.x * gi.y;
+      widths[lane] = gi.y;
+      mirrors[lane] = gi.w;
+      if (ok) {
+        own_shift[lane] = msh[rg.x];
+        mirror_shift[lane] = msh[mr.x];
+      }
+    }
+    if (lane == 0) {
+      first_column[nw] = width;
+      fast = ok;
+    }
+  }
+  __syncthreads();
+  if (!fast) {
+    for (int chunk = blockIdx.y; chunk < chunks; chunk += gridDim.y)
+      for (int w = warp; w < nw; w += kStripThreads / 32)
+        window_sums<V>(st.x + w, lane, chunk * kBlochKChunk,
+                       min(n_k - chunk * kBlochKChunk, kBlochKChunk), group, gdst, gmem, moff, msh,
+                       hv, sv, phases, n_shifts, nnz, hout, sout);
+    return;
+  }
+  const int4 g0 = group[st.x];
+  const int nr = g0.x, rl = g0.z;
+  if (warp < nw) {
+    const int ne = nr * widths[warp], v0 = first_value[warp];
+    const int64_t own = moff[gmem[st.x + warp].x], mir = moff[gmem[mirrors[warp]].x];
+    for (int e = lane; e < ne; e += 32) {
+      const V* src[4] = {hv + own + e, sv + own + e, hv + mir + e, sv + mir + e};
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(&vals[t / 2][t % 2][v0 + e])),
+                     "l"(src[t]), "n"(sizeof(V))
+                     : "memory");
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  // this thread's column: window, column in it, its value arrays
+  constexpr int kRowLanes = kStripThreads / kStripColumns;
+  const int col = threadIdx.x % kStripColumns, a0 = threadIdx.x / kStripColumns;
+  if (col >= first_column[nw]) return;
+  int w = 0;
+  while (col >= first_column[w + 1]) ++w;
+  const int c = col - first_column[w], nc = widths[w], g = st.x + w, gm = mirrors[w];
+  const V* own = &vals[0][0][first_value[w]];
+  const V* mir = &vals[1][0][first_value[w]];
+  const int64_t at0 = gdst[st.x] + col;
+  for (int chunk = blockIdx.y; chunk < chunks; chunk += gridDim.y) {
+    const int k0 = chunk * kBlochKChunk, nk = min(n_k - k0, kBlochKChunk);
+    const float2* ph0 = phases + (int64_t)k0 * n_shifts;
+    float2 po[kBlochKChunk], pm[kBlochKChunk];
+#pragma unroll
+    for (int q = 0; q < kBlochKChunk; ++q) {
+      po[q] = q < nk ? ph0[q * n_shifts + own_shift[w]] : make_float2(0.0f, 0.0f);
+      pm[q] = q < nk ? ph0[q * n_shifts + mirror_shift[w]] : make_float2(0.0f, 0.0f);
+    }
+    for (int a = a0; a < nr; a += kRowLanes) {
+      const bool lower = gm < g || (gm == g && a > c);
+      const int64_t at = (int64_t)k0 * nnz + at0 + (int64_t)a * rl;
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const float2 vo = load_value<V>(own + m * kStripValues, a * nc + c);
+        const float2 vm = load_value<V>(mir + m * kStripValues, c * nr + a);
+        float2* out = (m == 0 ? hout : sout) + at;
+#pragma unroll
+        for (int q = 0; q < kBlochKChunk; ++q) {
+          if (q < nk) {
+            const float2 xo = cmul_rn(vo, po[q]), xm = cmul_rn(vm, pm[q]);
+            const float2 mean = lower ? hermitian_mean(xm, xo) : hermitian_mean(xo, xm);
+            float2 v = lower ? make_float2(mean.x, -mean.y) : mean;
+            if (gm == g && a == c) v = make_float2(xo.x, 0.0f);
+            out[q * nnz] = v;
+          }
+        }
       }
     }
   }
@@ -375,6 +435,23 @@ int aosb_bloch_create(int64_t n_orbitals, int64_t n_atoms, const int64_t* atom_o
     g_dst[g] = B->indptr[atom_offsets[i]] + colpos[g];
   }
   B->n_members = (int64_t)m_off.size();
+  // Strips of each row atom, of about equal window counts.
+  for (int64_t a = 0; a < n_atoms; ++a) {
+    const int64_t lo = first_group[a], hi = first_group[a + 1];
+    const int64_t most = std::max<int64_t>(1, (hi - lo + kStripWindows - 1) / kStripWindows);
+    const int64_t even = (hi - lo + most - 1) / most;
+    for (int64_t g = lo; g < hi;) {
+      int64_t e = g, cols = 0, values = 0;
+      while (e < hi && e - g < even) {
+        cols += g_info[e].y;
+        values += (int64_t)g_info[e].x * g_info[e].y;
+        if (e > g && (cols > kStripColumns || values > kStripValues)) break;
+        ++e;
+      }
+      B->strips.push_back(make_int2((int)g, (int)e));
+      g = e;
+    }
+  }
   B->g_info = std::move(g_info);
   B->g_dst = std::move(g_dst);
   B->g_mem = std::move(g_mem);
@@ -394,7 +471,8 @@ int aosb_bloch_upload(aosb_bloch_t* B, char* err, size_t cap) {
       (rc = upload(&B->d_group_dst, B->g_dst, err, cap)) ||
       (rc = upload(&B->d_group_members, B->g_mem, err, cap)) ||
       (rc = upload(&B->d_member_off, B->m_off, err, cap)) ||
-      (rc = upload(&B->d_member_shift, B->m_shift, err, cap)))
+      (rc = upload(&B->d_member_shift, B->m_shift, err, cap)) ||
+      (rc = upload(&B->d_strips, B->strips, err, cap)))
     return rc;
   int64_t values = 0;
   for (size_t g = 0; g < B->g_info.size(); ++g)
@@ -465,20 +543,24 @@ int aosb_bloch_apply(const aosb_bloch_t* b, int32_t value_kind, const void* h_va
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "call aosb_bloch_upload first");
   if (n_k <= 0 || n_k > 65535)
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "n_k must be in 1..65535");
-  const int warps = 8;
-  dim3 grid(aosb::ceil_div(b->n_groups, warps), aosb::ceil_div(n_k, kBlochKChunk));
+  // A CTA goes through all k chunks with its blocks loaded once, unless the
+  // strips alone leave SMs without eight CTAs.
+  const int64_t strips = (int64_t)b->strips.size();
+  const int64_t chunks = aosb::ceil_div(n_k, kBlochKChunk);
+  const int64_t share = std::min<int64_t>(chunks, std::max<int64_t>(1, 148 * 8 / strips));
+  dim3 grid((unsigned)strips, (unsigned)share);
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nsh = (int64_t)(b->shifts.size() / 3);
   cudaEvent_t ev[2];
   const bool timed = aosb::timing_begin(st, ev);
   if (value_kind == 0) {
-    bloch_windows_kernel<float><<<grid, warps * 32, 0, st>>>(
-        b->n_groups, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
+    bloch_strips_kernel<float><<<grid, kStripThreads, 0, st>>>(
+        b->d_strips, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
         b->d_member_shift, (const float*)h_values, (const float*)s_values,
         (const float2*)phases, nsh, b->nnz, n_k, (float2*)h_out, (float2*)s_out);
   } else if (value_kind == 1) {
-    bloch_windows_kernel<float2><<<grid, warps * 32, 0, st>>>(
-        b->n_groups, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
+    bloch_strips_kernel<float2><<<grid, kStripThreads, 0, st>>>(
+        b->d_strips, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
         b->d_member_shift, (const float2*)h_values, (const float2*)s_values,
         (const float2*)phases, nsh, b->nnz, n_k, (float2*)h_out, (float2*)s_out);
   } else {
@@ -491,7 +573,7 @@ int aosb_bloch_apply(const aosb_bloch_t* b, int32_t value_kind, const void* h_va
     aosb::timing_end(aosb::kTimedBloch, st, ev, 0.0,
                      (double)b->n_values * 2.0 * (value_kind ? 8.0 : 4.0) +
                          (double)n_k * (double)b->nnz * 2.0 * 8.0);
-  return aosb::launch_check(err, cap, "bloch_windows_kernel");
+  return aosb::launch_check(err, cap, "bloch_strips_kernel");
 }
 
 void aosb_bloch_destroy(aosb_bloch_t* b) {
@@ -503,6 +585,7 @@ void aosb_bloch_destroy(aosb_bloch_t* b) {
   cudaFree(b->d_group_members);
   cudaFree(b->d_member_off);
   cudaFree(b->d_member_shift);
+  cudaFree(b->d_strips);
   delete b;
 }
 
