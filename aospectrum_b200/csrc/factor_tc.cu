@@ -712,13 +712,14 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   // rest of step k's Schur update runs on the others.
   const bool lookahead = tc_panels && sms >= 32;
   const int chosen = g_lookahead_sms.load();
-  // default: 5/4 of the pencils (the side stream's diagonal LU runs one CTA
-  // per pencil), at most a third of the SMs; the reserved SMs join the rest
-  // of the two-step update once the panels are done, so a generous reserve
-  // costs little (c2: 48 SMs beat 37 at 64 pencils, 40 beat 24 and 16 at 32)
-  const int reserve = !lookahead ? 0
-                      : chosen > 0 ? std::min(chosen, sms / 2)
-                                   : std::min(std::max(np * 5 / 4, 8), sms / 3);
+  // default: a third of the SMs.  The side stream's chain (two diagonal LUs,
+  // three 128-deep updates of a tile row and column, four stagings) must not
+  // outlast the rest update, and the reserved SMs join that update once the
+  // chain is done, so a generous reserve costs little.  1000-atom cube, ms a
+  // factorization with 5/4 SM a pencil / a third: 1 pencil 23.4 / 17.3, 4: 51.4
+  // / 36.3, 8: 81.9 / 67.9, 16: 130.7 / 131.2, 32 and 64 alike; 343 atoms, 13
+  // orbitals, 4 pencils: 9.7 / 6.7.
+  const int reserve = !lookahead ? 0 : chosen > 0 ? std::min(chosen, sms / 2) : sms / 3;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_cross = nullptr, ev_panel = nullptr;
   if (lookahead) {
