@@ -232,24 +232,27 @@ struct PShared {
 //     k + 1, "cross" holds the pairs with a < a0 or b < b0 -- every target
 //     in tile row or column k + 1, which step k + 1's diagonal LU and panels
 //     read -- and "rest" the pairs with a >= a0 and b >= b0.
-//   kMapList: two-step (K = 256) Schur items from the plan's super-step
-//     lists: item = (target slot, A and B staged index of the first step or
-//     -1, of the second step or -1); the first step's tiles come from
-//     `staging`, the second's from `staging1`.
+//   kMapList: Schur items of `steps` (2 or 4) tile steps from the plan's
+//     lists: item = (target slot, then per step the A and B staged index or
+//     -1); step h's tiles come from the h-th staging buffer after `staging`.
 enum MapKind : int { kMapSchur = 0, kMapPanel = 1, kMapCross = 2, kMapRest = 3, kMapList = 4 };
 
 struct ItemMap {
-  int kind, nL, nU, n_pairs, a0, b0;
+  int kind, nL, nU, n_pairs, a0, b0, steps;
   const int32_t* tslot;  // Schur targets [nL * nU]
   const int32_t* lslot;  // panel L targets [nL]
   const int32_t* uslot;  // panel U targets [nU]
-  const int32_t* list;   // kMapList items [n_pairs][5]
+  const int32_t* list;   // kMapList items [n_pairs][1 + 2 * steps]
 };
 
-// K halves of an item: staged (A, B) indices and which staging buffer
-// (0 = `staging`, 1 = `staging1`); returns how many (1 or 2).
-__device__ __forceinline__ int item_halves(const ItemMap& m, int pair, int (&ia)[2], int (&ib)[2],
-                                           int (&buf)[2]);
+constexpr int kMaxSteps = 4;
+
+// The tile steps of an item that hold products: staged (A, B) indices and
+// the staging buffer of each.
+struct ItemSteps {
+  int n;
+  int a[kMaxSteps], b[kMaxSteps], buf[kMaxSteps];
+};
 
 __device__ __forceinline__ void item_pair(const ItemMap& m, int pair, int& a, int& b) {
   if (m.kind == kMapSchur) {
@@ -289,32 +292,38 @@ __device__ __forceinline__ void item_operands(const ItemMap& m, int pair, int& i
   ib = m.nL + b;
 }
 
-__device__ __forceinline__ int item_halves(const ItemMap& m, int pair, int (&ia)[2], int (&ib)[2],
-                                           int (&buf)[2]) {
+__device__ __forceinline__ void item_steps(const ItemMap& m, int pair, ItemSteps& it) {
+  it.n = 0;
   if (m.kind != kMapList) {
-    item_operands(m, pair, ia[0], ib[0]);
-    buf[0] = 0;
-    return 1;
+    item_operands(m, pair, it.a[0], it.b[0]);
+    it.buf[0] = 0;
+    it.n = 1;
+    return;
   }
-  const int32_t* e = m.list + (size_t)pair * 5;
-  int nh = 0;
-  if (e[1] >= 0) {
-    ia[nh] = e[1];
-    ib[nh] = e[2];
-    buf[nh] = 0;
-    ++nh;
+  const int32_t* e = m.list + (size_t)pair * (1 + 2 * m.steps) + 1;
+#pragma unroll
+  for (int s = 0; s < kMaxSteps; ++s) {
+    if (s < m.steps && e[2 * s] >= 0) {
+      it.a[it.n] = e[2 * s];
+      it.b[it.n] = e[2 * s + 1];
+      it.buf[it.n] = s;
+      ++it.n;
+    }
   }
-  if (e[3] >= 0) {
-    ia[nh] = e[3];
-    ib[nh] = e[4];
-    buf[nh] = 1;
-    ++nh;
-  }
-  return nh;
+}
+
+// How many of the item's steps hold products.
+__device__ __forceinline__ int item_step_count(const ItemMap& m, int pair) {
+  if (m.kind != kMapList) return 1;
+  const int32_t* e = m.list + (size_t)pair * (1 + 2 * m.steps) + 1;
+  int n = 0;
+#pragma unroll
+  for (int s = 0; s < kMaxSteps; ++s) n += s < m.steps && e[2 * s] >= 0 ? 1 : 0;
+  return n;
 }
 
 __device__ __forceinline__ int item_target(const ItemMap& m, int pair) {
-  if (m.kind == kMapList) return m.list[(size_t)pair * 5];
+  if (m.kind == kMapList) return m.list[(size_t)pair * (1 + 2 * m.steps)];
   if (m.kind == kMapPanel) return pair < m.nL ? m.lslot[pair] : m.uslot[pair - m.nL];
   int a, b;
   item_pair(m, pair, a, b);
@@ -323,7 +332,7 @@ __device__ __forceinline__ int item_target(const ItemMap& m, int pair) {
 
 __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
     const ItemMap map, int n_pencils, int64_t n_slots, const unsigned char* __restrict__ staging,
-    const unsigned char* __restrict__ staging1, int64_t staging_pencil_stride,
+    int64_t staging_step_stride, int64_t staging_pencil_stride,
     int32_t* __restrict__ status, int* __restrict__ claim,
     const __grid_constant__ CUtensorMap tmap_c, long long wl) {
   const int n_pairs = map.n_pairs;
@@ -371,8 +380,9 @@ __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
       // copies instead of draining the ring at every item boundary.  A
       // claimed item is always processed by the CTA that claimed it.
       int cur = claim != nullptr ? atomicAdd(claim, 1) : (int)blockIdx.x;
-      int ia[2], ib[2], bf[2], nh = 0;
-      if (cur < total) nh = item_halves(map, cur % n_pairs, ia, ib, bf);
+      ItemSteps now, next;
+      now.n = next.n = 0;
+      if (cur < total) item_steps(map, cur % n_pairs, now);
       int nxt = claim != nullptr ? atomicAdd(claim, 1) : cur + (int)gridDim.x;
       for (int j = 0; !sh.failed; ++j) {
         int it = cur < total ? cur : -1;
@@ -394,14 +404,17 @@ __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
           break;
         }
         const int p = it / n_pairs;
-        const int nslabs = nh * kSlabs;
-        int na[2] = {0, 0}, nb[2] = {0, 0}, nf[2] = {0, 0}, nnh = 0;
+        const int nslabs = now.n * kSlabs;
+        const unsigned char *stA = nullptr, *stB = nullptr;
         for (int s = 0; s < nslabs; ++s) {
-          if (s == 2 && nxt < total) nnh = item_halves(map, nxt % n_pairs, na, nb, nf);
+          if (s == 2 && nxt < total) item_steps(map, nxt % n_pairs, next);
           const int h = s / kSlabs, sl = s % kSlabs;
-          const unsigned char* base = (bf[h] ? staging1 : staging) + (size_t)p * staging_pencil_stride;
-          const unsigned char* stA = base + (size_t)ia[h] * kStagedTileBytes;
-          const unsigned char* stB = base + (size_t)ib[h] * kStagedTileBytes;
+          if (sl == 0) {
+            const unsigned char* base = staging + (size_t)now.buf[h] * staging_step_stride +
+                                        (size_t)p * staging_pencil_stride;
+            stA = base + (size_t)now.a[h] * kStagedTileBytes;
+            stB = base + (size_t)now.b[h] * kStagedTileBytes;
+          }
           if (!mbar_wait(&sh.empty[stage], phase ^ 1, wl)) {
             sh.failed = 1;
             atomicCAS(&status[p], 0, (int)AOSB_ERR_TIMEOUT);
@@ -418,12 +431,7 @@ __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
         }
         if (sh.failed) break;
         cur = nxt;
-        nh = nnh;
-        for (int q = 0; q < 2; ++q) {
-          ia[q] = na[q];
-          ib[q] = nb[q];
-          bf[q] = nf[q];
-        }
+        now = next;
         nxt = cur >= total ? total : claim != nullptr ? atomicAdd(claim, 1) : cur + (int)gridDim.x;
       }
     }
@@ -457,8 +465,7 @@ __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
           first_waited = true;
         }
         const int p = it / n_pairs;
-        int ia[2], ib[2], bf[2];
-        const int nslabs = item_halves(map, it % n_pairs, ia, ib, bf) * kSlabs;
+        const int nslabs = item_step_count(map, it % n_pairs) * kSlabs;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t re = tmem + (uint32_t)acc * 256, im = re + kTcT;
         bool ok = true;
@@ -618,14 +625,15 @@ static int64_t staged_tiles_per_pencil(const aosb_plan* P) {
   return most + 2;
 }
 
-// Four staging buffers (tile step k uses buffer k % 4): with two-step
-// updates and lookahead, steps k + 2 and k + 3 are staged while the
-// two-step update of steps k and k + 1 still reads theirs.  After them, 256
-// bytes hold the item counter of the shared two-step updates.
+// Staging buffers: the steps of two groups, since the next group is staged
+// while the update of the current one still reads its own -- four with
+// two-step updates, eight where the plan has four-step lists.  After them,
+// 256 bytes hold the item counter of the shared updates.
+static int stage_buffers(const aosb_plan* P) { return P->qs_items.empty() ? 4 : 2 * kMaxSteps; }
 constexpr size_t kClaimBytes = 256;
 size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils) {
   if (P->T != kTcT) return 0;
-  return 4 * (size_t)staged_tiles_per_pencil(P) * kStagedTileBytes * (size_t)n_pencils +
+  return stage_buffers(P) * (size_t)staged_tiles_per_pencil(P) * kStagedTileBytes * (size_t)n_pencils +
          kClaimBytes;
 }
 
@@ -738,7 +746,8 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     }
   } guard{ev_cross, ev_panel};
   const int64_t buffer_bytes = (int64_t)np * pencil_stride;
-  auto stage_buf = [&](int64_t k) { return staging + (k & 3) * buffer_bytes; };
+  const int n_buffers = stage_buffers(P);
+  auto stage_buf = [&](int64_t k) { return staging + (k % n_buffers) * buffer_bytes; };
 
   // diagonal LU + panel products of step k on stream s (panel grid <= cap_ctas)
   auto panels = [&](int64_t k, cudaStream_t s, int cap_ctas) -> int {
@@ -752,9 +761,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     stage_kernel<<<dim3(nL + nU + 2, np), 256, 0, s>>>(
         nL, nU, 1, (int)k, lslot, uslot, P->diag_slot[k], P->n_slots, P->n_pad, a->factor,
         a->pivots, stage_buf(k), pencil_stride);
-    const ItemMap pm{kMapPanel, nL, nU, nL + nU, 0, 0, nullptr, lslot, uslot, nullptr};
+    const ItemMap pm{kMapPanel, nL, nU, nL + nU, 0, 0, 1, nullptr, lslot, uslot, nullptr};
     schur_tc_kernel<<<grid_for((int64_t)(nL + nU) * np, cap_ctas), kPThreads, smem, s>>>(
-        pm, np, P->n_slots, stage_buf(k), stage_buf(k), pencil_stride, a->status, nullptr, tmap_c, wl);
+        pm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl);
     count_launches(2);
     return 0;
   };
@@ -774,10 +783,10 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
                       cudaStream_t s) {
     const int nL = P->lb_off[k + 1] - P->lb_off[k];
     const int nU = P->ur_off[k + 1] - P->ur_off[k];
-    const ItemMap sm{kind, nL, nU, n_pairs, a0, b0, P->d_sc_slot + P->sc_off[k], nullptr, nullptr,
+    const ItemMap sm{kind, nL, nU, n_pairs, a0, b0, 1, P->d_sc_slot + P->sc_off[k], nullptr, nullptr,
                      nullptr};
     schur_tc_kernel<<<grid_for((int64_t)n_pairs * np, cap_ctas), kPThreads, smem, s>>>(
-        sm, np, P->n_slots, stage_buf(k), stage_buf(k), pencil_stride, a->status, nullptr, tmap_c, wl);
+        sm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl);
     count_launches(1);
   };
   // Schur update of step k (the pairs `kind` selects) on the caller stream,
@@ -788,10 +797,10 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     const int64_t items = (int64_t)n_pairs * np;
     cudaEvent_t ev[2];
     const bool timed = timing_begin(st, ev);
-    const ItemMap sm{kind, nL, nU, n_pairs, a0, b0, P->d_sc_slot + P->sc_off[k], nullptr, nullptr,
+    const ItemMap sm{kind, nL, nU, n_pairs, a0, b0, 1, P->d_sc_slot + P->sc_off[k], nullptr, nullptr,
                      nullptr};
     schur_tc_kernel<<<grid_for(items, cap_ctas), kPThreads, smem, st>>>(
-        sm, np, P->n_slots, stage_buf(k), stage_buf(k), pencil_stride, a->status, nullptr, tmap_c, wl);
+        sm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl);
     count_launches(1);
     if (timed)
       timing_end(kTimedSchur, st, ev, (double)items * 8.0 * kTcT * kTcT * kTcT,
@@ -812,7 +821,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   // two-step update of super-step ss (tile steps 2 ss, 2 ss + 1), the cross
   // or the rest items, on stream s (timed); with `claim` the launch takes
   // items from the shared counter instead of a fixed share
-  int* claim_counter = reinterpret_cast<int*>(staging + 4 * (int64_t)np * pencil_stride);
+  int* claim_counter = reinterpret_cast<int*>(staging + n_buffers * buffer_bytes);
   const bool pairs = g_schur_pairs.load() != 0 && P->d_sp_rest != nullptr;
   int pair_rc = 0;
   auto two_step = [&](int64_t ss, bool cross, int cap_ctas, cudaStream_t s = nullptr,
@@ -834,15 +843,16 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
       const std::vector<int64_t>& poff = cross ? P->sp_cross_off : P->sp_rest_off;
       const int32_t* pdev = cross ? P->d_sp_cross : P->d_sp_rest;
       const int rc = schur_pair_launch(pdev + 8 * poff[ss], poff[ss + 1] - poff[ss], np,
-                                       P->n_slots, staging, 4 * buffer_bytes,
-                                       (k0 & 3) * buffer_bytes, ((k0 + 1) & 3) * buffer_bytes,
+                                       P->n_slots, staging, n_buffers * buffer_bytes,
+                                       (k0 % n_buffers) * buffer_bytes,
+                                       ((k0 + 1) % n_buffers) * buffer_bytes,
                                        pencil_stride, a->status, claim, tmap_c, cap_ctas, s, err,
                                        cap);
       if (rc != 0 && pair_rc == 0) pair_rc = rc;
     } else {
-      const ItemMap lm{kMapList, 0, 0, (int)n, 0, 0, nullptr, nullptr, nullptr, dev + 5 * off[ss]};
+      const ItemMap lm{kMapList, 0, 0, (int)n, 0, 0, 2, nullptr, nullptr, nullptr, dev + 5 * off[ss]};
       schur_tc_kernel<<<grid_for(n * np, cap_ctas), kPThreads, smem, s>>>(
-          lm, np, P->n_slots, stage_buf(k0), stage_buf(k0 + 1), pencil_stride, a->status, claim,
+          lm, np, P->n_slots, stage_buf(k0), buffer_bytes, pencil_stride, a->status, claim,
           tmap_c, wl);
       count_launches(1);
     }
@@ -867,6 +877,75 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   // super-step's two panels beside the rest.
   const bool two_steps = tc_panels && lookahead && a->precision == AOSB_PRECISION_BF16X3 &&
                          P->d_ss_rest != nullptr;
+  // Four-step (K <= 512) updates: the same scheme with groups of four steps.
+  // List `l` (plan.h) of group g on stream s.
+  auto four_step = [&](int64_t g, int l, int cap_ctas, cudaStream_t s, int* claim = nullptr,
+                       bool count_work = true) {
+    const int64_t i0 = P->qs_off[5 * g + l], i1 = P->qs_off[5 * g + l + 1];
+    const int64_t n = i1 - i0, k0 = kMaxSteps * g;
+    if (n == 0) return;
+    cudaEvent_t ev[2];
+    const bool timed = count_work && timing_begin(s, ev);
+    const ItemMap lm{kMapList, 0, 0, (int)n, 0, 0, kMaxSteps, nullptr, nullptr, nullptr,
+                     P->d_qs_items + (1 + 2 * kMaxSteps) * i0};
+    schur_tc_kernel<<<grid_for(n * np, cap_ctas), kPThreads, smem, s>>>(
+        lm, np, P->n_slots, stage_buf(k0), buffer_bytes, pencil_stride, a->status, claim, tmap_c, wl);
+    count_launches(1);
+    if (timed) {
+      double products = 0;
+      for (int64_t i = i0; i < i1; ++i)
+        for (int h = 0; h < kMaxSteps; ++h)
+          products += P->qs_items[(1 + 2 * kMaxSteps) * i + 1 + 2 * h] >= 0 ? 1 : 0;
+      const int64_t k1 = std::min<int64_t>(k0 + kMaxSteps, P->nb);
+      const double staged =
+          (double)(P->lb_off[k1] - P->lb_off[k0] + P->ur_off[k1] - P->ur_off[k0]);
+      timing_end(kTimedSchur, s, ev, products * np * 8.0 * kTcT * kTcT * kTcT,
+                 (double)n * np * 2.0 * 2 * kTcT * kTcT * sizeof(float) +
+                     staged * np * kStagedTileBytes);
+    }
+  };
+  // Four steps halve the traffic of the targets (1 MB in and out per target
+  // and four steps becomes 512 KB), which the power limit turns into tensor
+  // clocks: the two-step update of 32 pencils of 102 tiles runs at 1.47 GHz,
+  // this one at 1.5-1.7.  They also double the chain of panels beside each
+  // rest update, so that update has to be long: at least 10,000 tile products
+  // a step over all pencils.  Below 500 products a step and pencil the plan
+  // has no four-step lists: the targets next to the diagonal, which cannot
+  // wait for all four steps, are then too large a share.  ms a factorization,
+  // two steps / four (products a step and pencil x pencils): 1421 x 4: 33.8 /
+  // 34.2, x 8: 66.7 / 63.1, x 32: 257 / 241; 951 x 8: 33.3 / 34.1, x 16: 65.8 /
+  // 63.8, x 64: 260 / 246; 522 x 8: 16.0 / 17.0, x 24: 39.6 / 37.9; 3043 x 2:
+  // 62.7 / 60.5, x 8: 230 / 216; 301 x 64: 45.8 / 46.3; 195 x 64: 103.8 / 111.4.
+  const bool four_steps = two_steps && !pairs && P->d_qs_items != nullptr &&
+                          P->schur_updates * np >= 10000 * P->nb;
+  if (four_steps) {
+    const int64_t nb = P->nb;
+    // the group's panels and staging, each after the updates of the group's
+    // earlier steps to that step's tile row and column
+    auto prepare = [&](int64_t g, cudaStream_t s, int cap_ctas) -> int {
+      for (int m = 0; m < kMaxSteps; ++m) {
+        const int64_t k = kMaxSteps * g + m;
+        if (k >= nb) break;
+        if (m > 0) four_step(g, m - 1, cap_ctas, s, nullptr, false);
+        if (int rc = panels(k, s, cap_ctas)) return rc;
+        stage_schur(k, s);
+      }
+      return 0;
+    };
+    if (int rc = prepare(0, st, sms)) return rc;
+    for (int64_t g = 0; kMaxSteps * (g + 1) < nb; ++g) {
+      four_step(g, kMaxSteps - 1, sms, st);
+      AOSB_CUDA_TRY(cudaMemsetAsync(claim_counter, 0, sizeof(int), st), err, cap);
+      AOSB_CUDA_TRY(cudaEventRecord(ev_cross, st), err, cap);
+      AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_cross, 0), err, cap);
+      if (int rc = prepare(g + 1, side, reserve)) return rc;
+      four_step(g, kMaxSteps, sms - reserve, st, claim_counter, true);
+      four_step(g, kMaxSteps, reserve, side, claim_counter, false);
+      AOSB_CUDA_TRY(cudaEventRecord(ev_panel, side), err, cap);
+      AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev_panel, 0), err, cap);
+    }
+    return launch_check(err, cap, "tensor-core factorization");
+  }
   if (two_steps) {
     const int64_t nb = P->nb;
     if (int rc = panels(0, st, sms)) return rc;

@@ -331,13 +331,70 @@ void build_super_steps(aosb_plan* P) {
   }
 }
 
+// Four-step Schur item lists (see plan.h).  The targets of a group are
+// gathered row by row, so a group costs one pass over its (L, U) pairs.
+void build_quad_steps(aosb_plan* P) {
+  constexpr int kSteps = 4;
+  const int64_t nb = P->nb;
+  P->qs_off.assign(1, 0);
+  P->qs_items.clear();
+  struct Item {
+    int32_t j, e[2 * kSteps];
+  };
+  std::vector<Item> row;
+  std::vector<int32_t> at(nb, -1);  // column -> position in `row`
+  std::vector<int32_t> lists[kSteps + 1];
+  for (int64_t k0 = 0; k0 < nb; k0 += kSteps) {
+    const int steps = (int)std::min<int64_t>(kSteps, nb - k0);
+    int32_t next[kSteps];  // first L tile of each step not yet passed
+    for (int s = 0; s < steps; ++s) next[s] = P->lb_off[k0 + s];
+    for (auto& l : lists) l.clear();
+    for (;;) {
+      // next target row with an L tile in one of the steps
+      int32_t i = INT32_MAX;
+      for (int s = 0; s < steps; ++s)
+        if (next[s] < P->lb_off[k0 + s + 1]) i = std::min(i, P->lb_tile[next[s]]);
+      if (i == INT32_MAX) break;
+      row.clear();
+      for (int s = 0; s < steps; ++s) {
+        const int64_t k = k0 + s;
+        if (next[s] == P->lb_off[k + 1] || P->lb_tile[next[s]] != i) continue;
+        const int32_t a = next[s]++ - P->lb_off[k];
+        const int32_t nL = P->lb_off[k + 1] - P->lb_off[k], u = P->ur_off[k];
+        for (int32_t b = 0; b < P->ur_off[k + 1] - u; ++b) {
+          const int32_t j = P->ur_tile[u + b];
+          if (at[j] < 0) {
+            at[j] = (int32_t)row.size();
+            row.push_back({j, {-1, -1, -1, -1, -1, -1, -1, -1}});
+          }
+          int32_t* e = row[at[j]].e;
+          e[2 * s] = a;
+          e[2 * s + 1] = nL + b;
+        }
+      }
+      std::sort(row.begin(), row.end(), [](const Item& x, const Item& y) { return x.j < y.j; });
+      for (const Item& it : row) {
+        at[it.j] = -1;
+        const int64_t q = std::min(i, it.j) - k0;
+        std::vector<int32_t>& dst = lists[q < kSteps ? q - 1 : q < 2 * kSteps ? kSteps - 1 : kSteps];
+        dst.push_back(P->slot[(int64_t)i * nb + it.j]);
+        dst.insert(dst.end(), it.e, it.e + 2 * kSteps);
+      }
+    }
+    for (auto& l : lists) {
+      P->qs_items.insert(P->qs_items.end(), l.begin(), l.end());
+      P->qs_off.push_back((int64_t)P->qs_items.size() / (1 + 2 * kSteps));
+    }
+  }
+}
+
 void plan_free_device(aosb_plan* p) {
   int32_t** arrs[] = {&p->d_perm, &p->d_pinv, &p->d_slot, &p->d_lb_slot, &p->d_ur_slot,
                       &p->d_ua_slot, &p->d_ll_slot, &p->d_lb_tile, &p->d_ur_tile,
                       &p->d_ua_tile, &p->d_ll_tile, &p->d_lb_off, &p->d_ur_off,
                       &p->d_ua_off, &p->d_ll_off, &p->d_sc_slot, &p->d_diag_slot,
                       &p->d_indices, &p->d_ss_cross, &p->d_ss_rest, &p->d_sp_cross,
-                      &p->d_sp_rest};
+                      &p->d_sp_rest, &p->d_qs_items};
   for (int32_t** a : arrs) {
     if (*a) cudaFree(*a);
     *a = nullptr;
@@ -607,6 +664,8 @@ int aosb_plan_create(int64_t n, const int64_t* indptr, const int32_t* indices,
     P->tree_levels = mx + 1;
   }
   aosb::build_super_steps(P);
+  // four-step updates pay from 500 tile products a step on (factor_tc.cu)
+  if (P->T == 128 && P->schur_updates >= 500 * P->nb) aosb::build_quad_steps(P);
   P->h_indptr.assign(indptr, indptr + n + 1);
   P->h_indices.assign(indices, indices + nnz);
   *out = P;
@@ -622,6 +681,7 @@ int aosb_plan_upload(aosb_plan_t* P, char* err, size_t cap) {
   if (rc == 0 && !P->ss_rest.empty()) rc = aosb::up(&P->d_ss_rest, P->ss_rest, err, cap);
   if (rc == 0 && !P->sp_cross.empty()) rc = aosb::up(&P->d_sp_cross, P->sp_cross, err, cap);
   if (rc == 0 && !P->sp_rest.empty()) rc = aosb::up(&P->d_sp_rest, P->sp_rest, err, cap);
+  if (rc == 0 && !P->qs_items.empty()) rc = aosb::up(&P->d_qs_items, P->qs_items, err, cap);
   if (rc == 0) rc = aosb::up(&P->d_indices, P->h_indices, err, cap);
   if (rc != 0) {
     aosb::plan_free_device(P);

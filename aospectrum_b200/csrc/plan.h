@@ -40,6 +40,16 @@ struct aosb_plan {
   // their A tiles.
   std::vector<int64_t> sp_cross_off, sp_rest_off;  // [n_super + 1], in pairs
   std::vector<int32_t> sp_cross, sp_rest;
+  // Four-step (K <= 512) Schur updates, group g = tile steps 4g .. 4g+3: every
+  // target right of and below the group's first step, in five lists by its
+  // first index q = min(row, column): lists 0..2 hold q = 4g+1 .. 4g+3 with
+  // the steps before q (they come before step q's panels), list 3 ("cross")
+  // q = 4g+4 .. 4g+7 (read by the next group's panels) and list 4 ("rest")
+  // the others, with all four steps.  9 ints per item: target slot, then per
+  // step the staged A and B indices or -1.  List l of group g:
+  // [qs_off[5g + l], qs_off[5g + l + 1]).
+  std::vector<int64_t> qs_off;
+  std::vector<int32_t> qs_items;
   // Device copies.
   int32_t *d_perm = nullptr, *d_pinv = nullptr, *d_slot = nullptr;
   int32_t *d_lb_slot = nullptr, *d_ur_slot = nullptr, *d_ua_slot = nullptr, *d_ll_slot = nullptr;
@@ -48,6 +58,7 @@ struct aosb_plan {
   int32_t *d_sc_slot = nullptr, *d_diag_slot = nullptr;
   int32_t *d_ss_cross = nullptr, *d_ss_rest = nullptr;
   int32_t *d_sp_cross = nullptr, *d_sp_rest = nullptr;
+  int32_t* d_qs_items = nullptr;
   // Pattern copies for the shifted-value assembly (host and device).
   std::vector<int64_t> h_indptr;
   std::vector<int32_t> h_indices;
@@ -61,4 +72,5 @@ int plan_upload(aosb_plan* p, char* err, size_t cap);
 void plan_free_device(aosb_plan* p);
 void solve_graphs_forget(const aosb_plan* p);
 void build_super_steps(aosb_plan* p);
+void build_quad_steps(aosb_plan* p);
 }  // namespace aosb

@@ -312,7 +312,8 @@ typedef struct {
 
 size_t aosb_factor_bytes(const aosb_plan_t *plan, int32_t n_pencils);
 /* Tensor-core precisions: four staging buffers of split-BF16 panel tiles
- * plus 256 bytes for the item counter that the two-step update's main and
+ * (eight for plans of at least 500 tile products a step, which take four steps
+ * at a time) plus 256 bytes for the item counter that an update's main and
  * lookahead launches share; 0 for precision 0.  A workspace sized for
  * n_pencils serves any batch of at most n_pencils; one factorization at a
  * time per workspace. */
