@@ -17,16 +17,24 @@
 //      split in BF16 (x = hi + lo) and written into the peers' shared memory in
 //      fragment order: 16 bytes hold two rows of one column;
 //   3. X_k = Y, and X_i -= op(F) Y for the step's tiles, cut into units of 32
-//      rows dealt out over the CTAs.  Two warps take a 32 KB unit (16 rows
-//      each): A fragments of mma.sync.m16n8k16 are read from the FP32 tile and
-//      split in registers, three products per real product (hi hi + hi lo +
-//      lo hi), FP32 accumulation; -acc is added to X in L2 (one red.add per
-//      element and step, so the result does not depend on timing).
+//      rows dealt out over the CTAs.  Four warps take a 32 KB unit (16 rows and
+//      half of K each; the halves are added through shared memory): A fragments
+//      of mma.sync.m16n8k16 are read from the FP32 tile and split in registers,
+//      three products per real product (hi hi + hi lo + lo hi), FP32
+//      accumulation; -acc is added to X in L2 (one red.add per element and
+//      step, so the result does not depend on timing).
 // The legacy tensor path suits this: with 32 columns a tile needs 3.2 us of it
 // per SM and 3.0 us of the SM's share of HBM, and its operands need no pass
 // through shared memory in the tensor core's layout.  A warp owns all columns
 // of its rows so that the split of A, the larger part of the other
-// instructions, is done once.
+// instructions, is done once.  What bounds the update is the latency of these
+// instructions (a scheduler with two such warps issues every third cycle), so
+// twelve warps share the work, as many as 128 registers allow: 64 pencils of
+// 102 tile steps, 32 columns, take 119 us a step against 128 with eight warps
+// that hold all of K, 8 pencils 30.3 against 32.0.  Sixteen warps at 96
+// registers spill (122 to 167), a split by columns repeats the split of A (140),
+// and a deeper ring (five units), an earlier release of its slots or slots of
+// 8 KB gain nothing (124, 126, 137).
 //
 // All waits are bounded: a wait that gives up sets AOSB_ERR_TIMEOUT for the
 // pencil, the CTA leaves its loops, waits for its own copies in flight and
@@ -51,8 +59,10 @@ constexpr int kParts = kT / kUnitRows;                 // units of a tile
 constexpr int kUnitPlane = kUnitRows * kT * 4;         // bytes of one plane of a unit
 constexpr uint32_t kUnitBytes = 2 * kUnitPlane;        // 32 KB
 constexpr int kBox = 32 * 32 * 4;                      // one TMA box
-constexpr int kConsumers = 256, kGroups = 4;           // four groups of two warps
-constexpr int kThreads = kConsumers + 32;              // + the producer warp
+constexpr int kGroups = 3;                             // groups of four warps
+constexpr int kWarps = 4 * kGroups, kConsumers = kWarps * 32;
+constexpr int kDiagWarps = 8;                          // warps of the diagonal product
+constexpr int kThreads = kConsumers + 32;              // + the producer warp: 13, four a scheduler
 // Units in the ring.  Entry g of the ring lies in slot g % kStages but counts
 // on full barrier g % kFull: a group waits only for its own entries, and with
 // 16 barriers it can never be a phase behind or ahead of one.
@@ -88,7 +98,7 @@ struct Shape {
   static constexpr int kRows = kT / D;               // rows of Y per CTA
   static constexpr int kTR = kRows >= 16 ? 4 : 2;    // rows per thread in the diagonal product
   static constexpr int kRowGroups = kRows / (4 * kTR);
-  static constexpr int kSlices = 8 / kRowGroups;     // warps that share K
+  static constexpr int kSlices = kDiagWarps / kRowGroups;  // warps that share K
   // ring entries that hold the CTA's rows of D: 32 rows each
   static constexpr int kDUnits = kRows > kUnitRows ? kRows / kUnitRows : 1;
 };
@@ -162,6 +172,11 @@ __device__ __forceinline__ bool consumers_any(bool v) {
   return out != 0;
 }
 
+__device__ __forceinline__ void pair_sync(int id) {
+  __syncwarp();
+  asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(id) : "memory");
+}
+
 // Two floats as BF16 pairs, x = hi + lo.
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(x1), "f"(x0));
@@ -177,16 +192,16 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// acc = op(F) Y for the 16 rows m16 .. m16 + 15 of a unit and NB blocks of
-// eight columns.  `order` (conjugate backward sweep): row r of Y belongs to
-// row order[r] of F.
+// acc = op(F) Y for the 16 rows m16 .. m16 + 15 of a unit, one half of K and NB
+// blocks of eight columns.  `order` (conjugate backward sweep): row r of Y
+// belongs to row order[r] of F.
 template <bool ADJ, bool ORDER, int NB>
 __device__ __forceinline__ void unit_product(const unsigned char* slab, const unsigned char* y,
-                                             const int* order, int m16, int lane,
+                                             const int* order, int m16, int khalf, int lane,
                                              float (&re)[4][4], float (&im)[4][4]) {
   const int fg = lane / 4, ft = lane % 4;  // fragment row (column of B), k pair
 #pragma unroll 2
-  for (int kb = 0; kb < kT / 16; ++kb) {
+  for (int kb = khalf * (kT / 32); kb < (khalf + 1) * (kT / 32); ++kb) {
     uint32_t arh[4], arl[4], aih[4], ail[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
@@ -212,29 +227,6 @@ __device__ __forceinline__ void unit_product(const unsigned char* slab, const un
       split2(r0, r1, arh[f], arl[f]);
       split2(i0, i1, aih[f], ail[f]);
     }
-    uint4 b0[NB], b1[NB];  // (re_hi, re_lo, im_hi, im_lo) of k pairs ft and ft + 4
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      const unsigned char* at = y + (kb * 8 + ft) * kYPitch + (b * 8 + fg) * 16;
-      b0[b] = *reinterpret_cast<const uint4*>(at);
-      b1[b] = *reinterpret_cast<const uint4*>(at + 4 * kYPitch);
-    }
-    // 2 NB accumulators in turn
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      mma(re[b], arh, b0[b].x, b1[b].x);
-      mma(im[b], arh, b0[b].z, b1[b].z);
-    }
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      mma(re[b], arh, b0[b].y, b1[b].y);
-      mma(im[b], arh, b0[b].w, b1[b].w);
-    }
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      mma(re[b], arl, b0[b].x, b1[b].x);
-      mma(im[b], arl, b0[b].z, b1[b].z);
-    }
     // plain: re -= Fi Yi, im += Fi Yr; conjugate: re += Fi Yi, im -= Fi Yr
     uint32_t nih[4], nil[4];
 #pragma unroll
@@ -242,20 +234,43 @@ __device__ __forceinline__ void unit_product(const unsigned char* slab, const un
       nih[f] = aih[f] ^ 0x80008000u;
       nil[f] = ail[f] ^ 0x80008000u;
     }
+    // two blocks of columns at a time: four accumulators in turn
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      mma(re[b], ADJ ? aih : nih, b0[b].z, b1[b].z);
-      mma(im[b], ADJ ? nih : aih, b0[b].x, b1[b].x);
-    }
+    for (int b = 0; b < NB; b += 2) {
+      const bool two = b + 1 < NB;
+      const int c = two ? b + 1 : b;
+      uint4 y0[2], y1[2];  // (re_hi, re_lo, im_hi, im_lo) of k pairs ft and ft + 4
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      mma(re[b], ADJ ? aih : nih, b0[b].w, b1[b].w);
-      mma(im[b], ADJ ? nih : aih, b0[b].y, b1[b].y);
-    }
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      mma(re[b], ADJ ? ail : nil, b0[b].z, b1[b].z);
-      mma(im[b], ADJ ? nil : ail, b0[b].x, b1[b].x);
+      for (int h = 0; h < 2; ++h)
+        if (h == 0 || two) {
+          const unsigned char* at = y + (kb * 8 + ft) * kYPitch + ((b + h) * 8 + fg) * 16;
+          y0[h] = *reinterpret_cast<const uint4*>(at);
+          y1[h] = *reinterpret_cast<const uint4*>(at + 4 * kYPitch);
+        }
+      auto word = [](const uint4& v, int w) {
+        return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
+      };
+      // re += ar (word r of Y), im += ai (word i of Y)
+      auto both = [&](const uint32_t(&ar)[4], int r, const uint32_t(&ai)[4], int i) {
+        mma(re[b], ar, word(y0[0], r), word(y1[0], r));
+        mma(im[b], ai, word(y0[0], i), word(y1[0], i));
+        if (two) {
+          mma(re[c], ar, word(y0[1], r), word(y1[1], r));
+          mma(im[c], ai, word(y0[1], i), word(y1[1], i));
+        }
+      };
+      both(arh, 0, arh, 2);
+      both(arh, 1, arh, 3);
+      both(arl, 0, arl, 2);
+      if (ADJ) {
+        both(aih, 2, nih, 0);
+        both(aih, 3, nih, 1);
+        both(ail, 2, nil, 0);
+      } else {
+        both(nih, 2, aih, 0);
+        both(nih, 3, aih, 1);
+        both(nil, 2, ail, 0);
+      }
     }
   }
 }
@@ -292,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int steps = 2 * a.nb;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kFull; ++s) mbar_init(&sh.full[s], 1);
-    for (int s = 0; s < kStages; ++s) mbar_init(&sh.empty[s], 2);
+    for (int s = 0; s < kStages; ++s) mbar_init(&sh.empty[s], 4);
     mbar_init(&sh.bar_y, D);
     mbar_init(&sh.bar_x, C);
     sh.failed = 0;
@@ -349,7 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int32_t* pivots = a.pivots + (size_t)p * a.n_pad;
     float2* X = a.work + (size_t)p * a.n_pad * a.nrhs + c0;
     int g = 0;  // ring entry
-    const int group = warp / 2, m16 = (warp & 1) * 16;
+    const int group = warp / 4, m16 = (warp & 1) * 16, khalf = warp / 2 & 1;
     const uint32_t y_local = smem_u32(sh.y);
     auto entry_ready = [&](int e) {
       return mbar_wait(&sh.full[e % kFull], (uint32_t)(e / kFull) & 1u, a.limit);
@@ -363,26 +378,28 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int units = (sw.off[k + 1] - sw.off[k]) * kParts;
       const bool gather = !ADJ && fwd, scatter = ADJ && !fwd;
       bool ok = true;
-      constexpr int kPairs = (R / 2 + 7) / 8;  // row pairs per warp
+      constexpr int kPairs = (R / 2 + kWarps - 1) / kWarps;  // row pairs per warp
       float2 y[kPairs][2];
       if (scatter && tid < kT) sh.order[tid] = pv[tid];
       if (diagonal) {
         // rows of X_k this thread stages, through the row interchanges
-        int from[kT / 16];
+        constexpr int kStaged = (kT + kConsumers / 16 - 1) / (kConsumers / 16);
+        int from[kStaged];
 #pragma unroll
-        for (int t = 0; t < kT / 16; ++t) {
-          const int r = tid / 16 + 16 * t;
-          from[t] = gather ? pv[r] : r;
+        for (int t = 0; t < kStaged; ++t) {
+          const int r = tid / 16 + kConsumers / 16 * t;
+          from[t] = gather && r < kT ? pv[r] : r;
         }
         ok = s == 0 || cluster_wait(&sh.bar_x, phase ^ 1u, a.limit);
         const float2* Xk = X + (size_t)k * kT * a.nrhs;
         {
           const int c = 2 * (tid % 16);
-          float4 v[kT / 16];
+          float4 v[kStaged];
 #pragma unroll
-          for (int t = 0; t < kT / 16; ++t) {
+          for (int t = 0; t < kStaged; ++t) {
             const float2* src = Xk + (size_t)from[t] * a.nrhs + c;
             v[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tid / 16 + kConsumers / 16 * t >= kT) break;
             if (a.wide) {
               if (c < ncols) v[t] = __ldcg(reinterpret_cast<const float4*>(src));
             } else {
@@ -399,8 +416,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
           }
 #pragma unroll
-          for (int t = 0; t < kT / 16; ++t)
-            *reinterpret_cast<float4*>(&sh.x[tid / 16 + 16 * t][c]) = v[t];
+          for (int t = 0; t < kStaged; ++t)
+            if (tid / 16 + kConsumers / 16 * t < kT)
+              *reinterpret_cast<float4*>(&sh.x[tid / 16 + kConsumers / 16 * t][c]) = v[t];
         }
 #pragma unroll
         for (int d = 0; d < S::kDUnits; ++d) ok = ok && entry_ready(g + d);
@@ -424,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 1
-          for (int q = slice * KS; q < (slice + 1) * KS; q += 4) {
+          for (int q = slice * KS; q < (slice + 1) * KS && warp < kDiagWarps; q += 4) {
             if (lower ? q > row + TR - 1 : q + 3 < row) continue;  // outside the triangle
             float dr[4][TR], di[4][TR];  // [k][row]
             if (!ADJ) {
@@ -483,12 +501,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
           }
           consumers_any(false);  // X_k and D are read: their space is free
-          if (warp < 2 && lane == 0)
+          if (warp < 4 && lane == 0)
 #pragma unroll
             for (int d = 0; d < S::kDUnits; ++d) mbar_arrive(&sh.empty[(g + d) % kStages]);
           float2(*part)[kStrip] = sh.x;  // [slice * R + row]
 #pragma unroll
-          for (int i = 0; i < TR; ++i) {
+          for (int i = 0; i < TR && warp < kDiagWarps; ++i) {
             float2* to = part[slice * R + rg + i];
             *reinterpret_cast<float4*>(&to[cg]) =
                 make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
@@ -501,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // sums of the partials for two rows of one column, to every peer
 #pragma unroll
         for (int o = 0; o < kPairs; ++o) {
-          const int i = 2 * (warp + 8 * o);
+          const int i = 2 * (warp + kWarps * o);
           if (i >= R) break;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -528,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ok = cluster_wait(&sh.bar_y, phase, a.limit);
 #pragma unroll
       for (int o = 0; o < kPairs; ++o) {
-        const int i = 2 * (warp + 8 * o);
+        const int i = 2 * (warp + kWarps * o);
         if (!diagonal || i >= R || lane >= ncols) break;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -538,9 +556,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       // update units of this CTA, in turn to the groups of warps
       for (int u = rank, j = 0; u < units; u += C, ++g, ++j) {
-        if ((j & (kGroups - 1)) != group) continue;
+        if (j % kGroups != group) continue;
         ok = ok && __all_sync(0xffffffffu, entry_ready(g) ? 1 : 0);
-        if (!ok) continue;
+        // after a failure both warps of a pair still meet
+        if (!ok) {
+          pair_sync(2 + group * 2 + (warp & 1));
+          pair_sync(2 + group * 2 + (warp & 1));
+          continue;
+        }
         const int row = sh.tile[g % kFull] + m16 + lane / 4;
         const unsigned char* slab = sh.ring[g % kStages];
         float re[4][4], im[4][4];
@@ -549,27 +572,45 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int e = 0; e < 4; ++e) re[b][e] = im[b][e] = 0.0f;
         if (ncols <= 8)
-          scatter ? unit_product<ADJ, ADJ, 1>(slab, sh.y, sh.order, m16, lane, re, im)
-                  : unit_product<ADJ, false, 1>(slab, sh.y, nullptr, m16, lane, re, im);
+          scatter ? unit_product<ADJ, ADJ, 1>(slab, sh.y, sh.order, m16, khalf, lane, re, im)
+                  : unit_product<ADJ, false, 1>(slab, sh.y, nullptr, m16, khalf, lane, re, im);
         else if (ncols <= 16)
-          scatter ? unit_product<ADJ, ADJ, 2>(slab, sh.y, sh.order, m16, lane, re, im)
-                  : unit_product<ADJ, false, 2>(slab, sh.y, nullptr, m16, lane, re, im);
+          scatter ? unit_product<ADJ, ADJ, 2>(slab, sh.y, sh.order, m16, khalf, lane, re, im)
+                  : unit_product<ADJ, false, 2>(slab, sh.y, nullptr, m16, khalf, lane, re, im);
         else if (ncols <= 24)
-          scatter ? unit_product<ADJ, ADJ, 3>(slab, sh.y, sh.order, m16, lane, re, im)
-                  : unit_product<ADJ, false, 3>(slab, sh.y, nullptr, m16, lane, re, im);
+          scatter ? unit_product<ADJ, ADJ, 3>(slab, sh.y, sh.order, m16, khalf, lane, re, im)
+                  : unit_product<ADJ, false, 3>(slab, sh.y, nullptr, m16, khalf, lane, re, im);
         else
-          scatter ? unit_product<ADJ, ADJ, 4>(slab, sh.y, sh.order, m16, lane, re, im)
-                  : unit_product<ADJ, false, 4>(slab, sh.y, nullptr, m16, lane, re, im);
+          scatter ? unit_product<ADJ, ADJ, 4>(slab, sh.y, sh.order, m16, khalf, lane, re, im)
+                  : unit_product<ADJ, false, 4>(slab, sh.y, nullptr, m16, khalf, lane, re, im);
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.empty[g % kStages]);
+        // The two warps of a row half add up: each hands over the blocks that
+        // the other one subtracts from X (the first half of K the low ones).
+        const int blocks = (ncols + 7) / 8, low = (blocks + 1) / 2;
+        float4* out = reinterpret_cast<float4*>(&sh.x[0][0]) + warp * 128 + lane;
+        const float4* in = reinterpret_cast<float4*>(&sh.x[0][0]) + (warp ^ 2) * 128 + lane;
+        pair_sync(2 + group * 2 + (warp & 1));  // the peer has read its last ones
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (b < blocks && (b < low) == (khalf == 1)) {
+            const int to = b < low ? b : b - low;
+            out[to * 64] = make_float4(re[b][0], re[b][1], re[b][2], re[b][3]);
+            out[to * 64 + 32] = make_float4(im[b][0], im[b][1], im[b][2], im[b][3]);
+          }
+        pair_sync(2 + group * 2 + (warp & 1));
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
           const int c = b * 8 + 2 * (lane % 4);
+          if (b >= blocks || (b < low) != (khalf == 0)) continue;
+          const int at = b < low ? b : b - low;
+          const float4 r = in[at * 64], m = in[at * 64 + 32];
           if (c >= ncols) continue;
           float2* to = X + (size_t)row * a.nrhs + c;
-          subtract(to, re[b][0], im[b][0], re[b][1], im[b][1], a.wide, c + 1 < ncols);
-          subtract(to + (size_t)8 * a.nrhs, re[b][2], im[b][2], re[b][3], im[b][3], a.wide,
+          subtract(to, re[b][0] + r.x, im[b][0] + m.x, re[b][1] + r.y, im[b][1] + m.y, a.wide,
                    c + 1 < ncols);
+          subtract(to + (size_t)8 * a.nrhs, re[b][2] + r.z, im[b][2] + m.z, re[b][3] + r.w,
+                   im[b][3] + m.w, a.wide, c + 1 < ncols);
         }
       }
       if (consumers_any(!ok)) {
@@ -666,15 +707,15 @@ Residency residency(int device) {
 // the diagonal product over its CTAs, the update units of the busiest CTA, all
 // times the waves of clusters. Fitted to whole
 // solves of the 1000- and 64-atom bundles (102 and 7 tile steps; us a step,
-// 32 columns, this kernel / one launch per step): 8 pencils 32 / 41, 16: 49 /
-// 56, 32: 67 / 84, 64: 127 / 142; 64 atoms, 5 pencils 10 / 32, 16: 16 / 42.
-// Past two waves of the smallest clusters the separate launches, which share
-// all units out over all SMs, win again (96 pencils: 257 / 200).
+// 32 columns, this kernel / one launch per step): 8 pencils 30 / 41, 16: 47 /
+// 56, 32: 63 / 84, 64: 119 / 142; 64 atoms, 5 pencils 10 / 32, 16: 16 / 42.
+// Past one wave of the smallest clusters the separate launches, which share
+// all units out over all SMs, win again (96 pencils: 240 / 200).
 double step_cost(const Form& f, int resident, int units, double tiles, int columns) {
   if (resident <= 0) return 1e30;
   const double waves = (units + resident - 1) / resident;
   const double rows = kT / f.diagonal;
-  const double unit = 0.4 + 0.29 * ((columns + 7) / 8);
+  const double unit = 0.45 + 0.24 * ((columns + 7) / 8);
   return waves * (6.5 + 0.15 * rows + unit * kParts * tiles / f.cluster);
 }
 
