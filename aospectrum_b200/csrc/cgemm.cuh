@@ -37,7 +37,9 @@ struct CgemmSmem {
 // A_MN: consecutive threads fetch consecutive rows m of A (for operands
 // read from a transposed tile, so that a warp reads along memory); by
 // default consecutive threads fetch consecutive k.
-template <int BM, int BN, int TM, int TN, bool A_MN = false, typename LoadA, typename LoadB>
+// REAL: the imaginary parts of both operands are zero and are left out.
+template <int BM, int BN, int TM, int TN, bool A_MN = false, bool REAL = false, typename LoadA,
+          typename LoadB>
 __device__ __forceinline__ void cgemm_cta(float (&accr)[TM][TN], float (&acci)[TM][TN], int K,
                                           CgemmSmem<BM, BN> (&sm)[2], LoadA loadA, LoadB loadB) {
   using S = CgemmShape<BM, BN, TM, TN>;
@@ -69,7 +71,7 @@ __device__ __forceinline__ void cgemm_cta(float (&accr)[TM][TN], float (&acci)[T
       if (e < BM * BK) {
         const int m = A_MN ? e % BM : e / BK, kk = A_MN ? e / BM : e % BK;
         buf.ar[kk][m] = ra[t].x;
-        buf.ai[kk][m] = ra[t].y;
+        if (!REAL) buf.ai[kk][m] = ra[t].y;
       }
     }
 #pragma unroll
@@ -77,7 +79,7 @@ __device__ __forceinline__ void cgemm_cta(float (&accr)[TM][TN], float (&acci)[T
       const int e = tid + t * 256;
       if (e < BK * BN) {
         buf.br[e / BN][e % BN] = rb[t].x;
-        buf.bi[e / BN][e % BN] = rb[t].y;
+        if (!REAL) buf.bi[e / BN][e % BN] = rb[t].y;
       }
     }
   };
@@ -95,18 +97,19 @@ __device__ __forceinline__ void cgemm_cta(float (&accr)[TM][TN], float (&acci)[T
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
         a_r[i] = b.ar[kk][tr * TM + i];
-        a_i[i] = b.ai[kk][tr * TM + i];
+        if (!REAL) a_i[i] = b.ai[kk][tr * TM + i];
       }
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         b_r[j] = b.br[kk][tc + j * S::kColThreads];
-        b_i[j] = b.bi[kk][tc + j * S::kColThreads];
+        if (!REAL) b_i[j] = b.bi[kk][tc + j * S::kColThreads];
       }
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
           accr[i][j] = fmaf(a_r[i], b_r[j], accr[i][j]);
+          if (REAL) continue;
           accr[i][j] = fmaf(-a_i[i], b_i[j], accr[i][j]);
           acci[i][j] = fmaf(a_r[i], b_i[j], acci[i][j]);
           acci[i][j] = fmaf(a_i[i], b_r[j], acci[i][j]);

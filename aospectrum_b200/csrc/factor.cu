@@ -84,7 +84,8 @@ struct PanelCfg {
   static_assert((T / UTM) * (32 / UTN) == 256, "U panel layout");
 };
 
-template <int T>
+// REAL: the factor's imaginary planes are zero and stay so (real pencils).
+template <int T, bool REAL>
 __global__ void __launch_bounds__(kThreads) panel_kernel(int k, int nL, int nU,
                                                          const int32_t* __restrict__ lslot,
                                                          const int32_t* __restrict__ uslot,
@@ -109,21 +110,21 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(int k, int nL, int nU,
     const int r0 = strip * S;
     auto la = [&](int m, int q) {
       const size_t o = (size_t)(r0 + m) * T + q;
-      return make_float2(A[o], A[o + T * T]);
+      return make_float2(A[o], REAL ? 0.f : A[o + T * T]);
     };
     auto lb = [&](int q, int c) {
       if (q > c) return make_float2(0.f, 0.f);
       const size_t o = (size_t)q * T + c;
-      return make_float2(D[o], D[o + T * T]);
+      return make_float2(D[o], REAL ? 0.f : D[o + T * T]);
     };
-    cgemm_cta<S, T, TM, TN>(accr, acci, T, sm, la, lb);
+    cgemm_cta<S, T, TM, TN, false, REAL>(accr, acci, T, sm, la, lb);
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         const size_t o = (size_t)(r0 + cg_row<S, T, TM, TN>(i)) * T + cg_col<S, T, TM, TN>(j);
         A[o] = accr[i][j];
-        A[o + T * T] = acci[i][j];
+        if (!REAL) A[o + T * T] = acci[i][j];
       }
   } else if (item < nL + nU) {
     // columns [strip*S, +S) of inv(L_kk) (P_k A_kj)
@@ -137,20 +138,20 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(int k, int nL, int nU,
       if (q > r) return make_float2(0.f, 0.f);
       if (q == r) return make_float2(1.f, 0.f);
       const size_t o = (size_t)r * T + q;
-      return make_float2(D[o], D[o + T * T]);
+      return make_float2(D[o], REAL ? 0.f : D[o + T * T]);
     };
     auto lb = [&](int q, int c) {
       const size_t o = (size_t)pv[q] * T + c0 + c;
-      return make_float2(A[o], A[o + T * T]);
+      return make_float2(A[o], REAL ? 0.f : A[o + T * T]);
     };
-    cgemm_cta<T, S, TM, TN>(accr, acci, T, sm, la, lb);
+    cgemm_cta<T, S, TM, TN, false, REAL>(accr, acci, T, sm, la, lb);
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         const size_t o = (size_t)cg_row<T, S, TM, TN>(i) * T + c0 + cg_col<T, S, TM, TN>(j);
         A[o] = accr[i][j];
-        A[o + T * T] = acci[i][j];
+        if (!REAL) A[o + T * T] = acci[i][j];
       }
   }
 }
@@ -210,10 +211,15 @@ __global__ void __launch_bounds__(kThreads) schur_words_kernel(
 // former 4 x 4 form with scalar words and slices staged through registers ran
 // at a third of the FP32 rate: 8 pencils of the 343-atom cube (5 orbitals) 88
 // us a step, now 72; 70 tiles of 64, one pencil: 71 us, now 59.
-constexpr int kSchurThreads = 128, kSchurK = 16, kSchurAPitch = kSchurK + 4;
+// Real pencils (the imaginary planes are zero and stay so) take a quarter of
+// the FMAs on half the data, in slices of 32 deep, with the same results to the
+// bit: 70 tiles of 64, one pencil, REAL_US us instead of 59.
+constexpr int kSchurThreads = 128;
+template <bool REAL>
 struct SchurSlice {
-  float a[2][64][kSchurAPitch];  // planes of L rows
-  float b[2][kSchurK][64];       // planes of U rows
+  static constexpr int kPlanes = REAL ? 1 : 2, kDepth = REAL ? 32 : 16;
+  float a[kPlanes][64][kDepth + 4];  // planes of L rows
+  float b[kPlanes][kDepth][64];      // planes of U rows
 };
 
 __device__ __forceinline__ void copy16(float* dst, const float* src) {
@@ -223,12 +229,13 @@ __device__ __forceinline__ void copy16(float* dst, const float* src) {
                : "memory");
 }
 
-template <int T>
+template <int T, bool REAL>
 __global__ void __launch_bounds__(kSchurThreads, 4) schur_kernel(
     int nU, const int32_t* __restrict__ lslot, const int32_t* __restrict__ uslot,
     const int32_t* __restrict__ tslot, int64_t n_slots, float* __restrict__ factor) {
-  constexpr int kParts = T / 64;
-  __shared__ __align__(16) SchurSlice sm[2];
+  using Slice = SchurSlice<REAL>;
+  constexpr int kParts = T / 64, kDepth = Slice::kDepth, I = Slice::kPlanes - 1;
+  __shared__ __align__(16) Slice sm[2];
   const int p = blockIdx.y;
   const int pair = blockIdx.x / (kParts * kParts), part = blockIdx.x % (kParts * kParts);
   const int m0 = part / kParts * 64, n0 = part % kParts * 64;
@@ -237,14 +244,14 @@ __global__ void __launch_bounds__(kSchurThreads, 4) schur_kernel(
   const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16 * 4;
   auto fetch = [&](int buf, int k0) {
 #pragma unroll
-    for (int plane = 0; plane < 2; ++plane) {
+    for (int plane = 0; plane < Slice::kPlanes; ++plane) {
 #pragma unroll
-      for (int e = tid; e < 64 * (kSchurK / 4); e += kSchurThreads) {
-        const int m = e / (kSchurK / 4), k = e % (kSchurK / 4) * 4;
+      for (int e = tid; e < 64 * (kDepth / 4); e += kSchurThreads) {
+        const int m = e / (kDepth / 4), k = e % (kDepth / 4) * 4;
         copy16(&sm[buf].a[plane][m][k], L + plane * T * T + m * T + k0 + k);
       }
 #pragma unroll
-      for (int e = tid; e < kSchurK * 16; e += kSchurThreads) {
+      for (int e = tid; e < kDepth * 16; e += kSchurThreads) {
         const int k = e / 16, n = e % 16 * 4;
         copy16(&sm[buf].b[plane][k][n], U + plane * T * T + (k0 + k) * T + n);
       }
@@ -257,33 +264,39 @@ __global__ void __launch_bounds__(kSchurThreads, 4) schur_kernel(
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
   fetch(0, 0);
-  for (int k0 = 0; k0 < T; k0 += kSchurK) {
-    const int buf = k0 / kSchurK & 1;
-    if (k0 + kSchurK < T) {
-      fetch(buf ^ 1, k0 + kSchurK);
+  for (int k0 = 0; k0 < T; k0 += kDepth) {
+    const int buf = k0 / kDepth & 1;
+    if (k0 + kDepth < T) {
+      fetch(buf ^ 1, k0 + kDepth);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    const SchurSlice& s = sm[buf];
+    const Slice& s = sm[buf];
 #pragma unroll
-    for (int k = 0; k < kSchurK; k += 4) {
+    for (int k = 0; k < kDepth; k += 4) {
       float4 br[4], bi[4];
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         br[h] = *reinterpret_cast<const float4*>(&s.b[0][k + h][tc]);
-        bi[h] = *reinterpret_cast<const float4*>(&s.b[1][k + h][tc]);
+        if (!REAL) bi[h] = *reinterpret_cast<const float4*>(&s.b[I][k + h][tc]);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float4 ar = *reinterpret_cast<const float4*>(&s.a[0][tr + 8 * i][k]);
-        const float4 ai = *reinterpret_cast<const float4*>(&s.a[1][tr + 8 * i][k]);
+        float4 ai;
+        if (!REAL) ai = *reinterpret_cast<const float4*>(&s.a[I][tr + 8 * i][k]);
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           const float re = h == 0 ? ar.x : h == 1 ? ar.y : h == 2 ? ar.z : ar.w;
-          const float im = h == 0 ? ai.x : h == 1 ? ai.y : h == 2 ? ai.z : ai.w;
           const float xr[4] = {br[h].x, br[h].y, br[h].z, br[h].w};
+          if (REAL) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j].x = fmaf(re, xr[j], acc[i][j].x);
+            continue;
+          }
+          const float im = h == 0 ? ai.x : h == 1 ? ai.y : h == 2 ? ai.z : ai.w;
           const float xi[4] = {bi[h].x, bi[h].y, bi[h].z, bi[h].w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -304,18 +317,20 @@ __global__ void __launch_bounds__(kSchurThreads, 4) schur_kernel(
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     float4* re = reinterpret_cast<float4*>(C + (tr + 8 * i) * T + tc);
-    float4* im = reinterpret_cast<float4*>(C + (tr + 8 * i) * T + tc + T * T);
-    float4 r = *re, m = *im;
+    float4 r = *re;
     r.x -= acc[i][0].x; r.y -= acc[i][1].x; r.z -= acc[i][2].x; r.w -= acc[i][3].x;
-    m.x -= acc[i][0].y; m.y -= acc[i][1].y; m.z -= acc[i][2].y; m.w -= acc[i][3].y;
     *re = r;
+    if (REAL) continue;
+    float4* im = re + T * T / 4;
+    float4 m = *im;
+    m.x -= acc[i][0].y; m.y -= acc[i][1].y; m.z -= acc[i][2].y; m.w -= acc[i][3].y;
     *im = m;
   }
 }
 
 template <int T>
 int launch_schur(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k, int nL, int nU,
-                 char* err, size_t cap) {
+                 bool real, char* err, size_t cap) {
   constexpr int parts = SchurCfg<T>::kSub;
   const int64_t blocks = (int64_t)nL * nU * parts;
   if (blocks > INT32_MAX) return set_error(err, cap, AOSB_ERR_SIZE, "schur grid too large");
@@ -326,7 +341,8 @@ int launch_schur(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k, in
   count_launches(1);
   if constexpr (T >= 64) {
     if (((uintptr_t)a->factor & 15) == 0) {
-      schur_kernel<T><<<grid, kSchurThreads, 0, st>>>(nU, l, u, t, P->n_slots, a->factor);
+      const auto kernel = real ? schur_kernel<T, true> : schur_kernel<T, false>;
+      kernel<<<grid, kSchurThreads, 0, st>>>(nU, l, u, t, P->n_slots, a->factor);
       return 0;
     }
   }
@@ -355,7 +371,7 @@ int ensure_diag_attr(char* err, size_t cap) {
 // Diagonal LU and panel updates of step k (FP32 SIMT).
 template <int T>
 void step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k,
-                 float* diag_tiles = nullptr) {
+                 bool real = false, float* diag_tiles = nullptr) {
   cudaStream_t st = (cudaStream_t)a->stream;
   const int np = a->n_pencils;
   const size_t diag_smem = diag_smem_bytes<T>();
@@ -366,23 +382,24 @@ void step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k,
   const int nU = P->ur_off[k + 1] - P->ur_off[k];
   if (nL + nU > 0) {
     dim3 grid((unsigned)((nL + nU) * PanelCfg<T>::kStrips), np);
-    panel_kernel<T><<<grid, kThreads, 0, st>>>((int)k, nL, nU, P->d_lb_slot + P->lb_off[k],
-                                               P->d_ur_slot + P->ur_off[k], P->d_diag_slot,
-                                               P->n_slots, P->n_pad, a->factor, a->pivots);
+    const auto kernel = real ? panel_kernel<T, true> : panel_kernel<T, false>;
+    kernel<<<grid, kThreads, 0, st>>>((int)k, nL, nU, P->d_lb_slot + P->lb_off[k],
+                                      P->d_ur_slot + P->ur_off[k], P->d_diag_slot, P->n_slots,
+                                      P->n_pad, a->factor, a->pivots);
     count_launches(1);
   }
 }
 
 template <int T>
-int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
+int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap, bool real,
               float* diag_tiles) {
   if (int rc = ensure_diag_attr<T>(err, cap)) return rc;
   for (int64_t k = 0; k < P->nb; ++k) {
-    step_panels<T>(P, a, k, diag_tiles);
+    step_panels<T>(P, a, k, real, diag_tiles);
     const int nL = P->lb_off[k + 1] - P->lb_off[k];
     const int nU = P->ur_off[k + 1] - P->ur_off[k];
     if (nL > 0 && nU > 0)
-      if (int rc = launch_schur<T>(P, a, k, nL, nU, err, cap)) return rc;
+      if (int rc = launch_schur<T>(P, a, k, nL, nU, real, err, cap)) return rc;
   }
   return launch_check(err, cap, "plain factorization");
 }
@@ -426,12 +443,12 @@ int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cu
   return 0;
 }
 
-int factor_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
+int factor_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap, bool real,
                  float* diag_tiles) {
   switch (P->T) {
-    case 32: return run_plain<32>(P, a, err, cap, diag_tiles);
-    case 64: return run_plain<64>(P, a, err, cap, diag_tiles);
-    case 128: return run_plain<128>(P, a, err, cap, diag_tiles);
+    case 32: return run_plain<32>(P, a, err, cap, real, diag_tiles);
+    case 64: return run_plain<64>(P, a, err, cap, real, diag_tiles);
+    case 128: return run_plain<128>(P, a, err, cap, real, diag_tiles);
   }
   return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "unsupported tile size");
 }

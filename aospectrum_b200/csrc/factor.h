@@ -11,11 +11,12 @@ int factor_step_panels(const aosb_plan* P, const aosb_factor_args_v1* a, int k, 
                        size_t cap);
 int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cudaStream_t st,
                      char* err, size_t cap);
-// `diag_tiles`, if given (T^2 floats per tile step): the real plane of pencil
+// `real`: all values and shifts are real, so the factor's imaginary planes are
+// zero and need no work.  `diag_tiles`, if given (T^2 floats per tile step): the real plane of pencil
 // 0's diagonal tile of each step as its LU found it, that is, the Schur
 // complement that the steps before left.
 int factor_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
-                 float* diag_tiles = nullptr);
+                 bool real = false, float* diag_tiles = nullptr);
 int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap);
 size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils);
 // Two-CTA (M = 256) Schur update of one pair list (schur_pair.cu): the

@@ -334,7 +334,7 @@ int factorize(aosb_shift_factor* f, float shift, char* err, size_t cap) {
                          f->d_factor, f->d_piv, f->d_status, nullptr, f->stream};
   if (int rc = inertia_attributes((int)P->T, err, cap)) return rc;
   if (int rc = factor_assemble(P, &fa, err, cap)) return rc;
-  if (int rc = factor_plain(P, &fa, err, cap, f->d_tiles)) return rc;
+  if (int rc = factor_plain(P, &fa, err, cap, true, f->d_tiles)) return rc;
   if (int rc = tile_inertias(f, err, cap)) return rc;
   int32_t counts[4] = {0, 0, 0, 0}, status = 0;
   AOSB_CUDA_TRY(cudaMemcpyAsync(counts, f->d_counts, sizeof(counts), cudaMemcpyDeviceToHost,
