@@ -251,6 +251,364 @@ __global__ void __launch_bounds__(kThreads) solve_update_kernel(
     }
 }
 
+// FP32 sweeps (no tensor cores), two kernels a step: Y = op(D_kk) X_k in blocks
+// of 16 rows, then X_i -= op(F) Y in blocks of 32 rows, 32 columns each.  With
+// tens of tiles a step these are latency chains: launch, operand loads, product,
+// store.  So the blocks are small (the product takes half a microsecond), all
+// loads of a block are in flight together, and each kernel is launched
+// programmatically: it starts while the one before it ends and fetches its part
+// of the factor before it waits for that one's results.  The first kernel of a
+// solve is launched in the ordinary way, so that the factor is complete.
+// Microseconds a step, against blocks of 32 and 64 rows with operands through
+// registers in slices of 16 and full waits between the launches: 343 atoms (27
+// steps of 64, 32 columns) 1 pencil 6 / 17, 8: 12.5 / 21.5, 64: 27 / 43, 128: 47
+// / 69; 26 steps of 32, 8 pencils 5 / 12; 102 steps of 128, 8 pencils 39 / 59,
+// 32: 118 / 156.
+constexpr int kRowsThreads = 128;
+
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// 16 (8) bytes to shared memory, zeros if `have` is false.
+__device__ __forceinline__ void copy_async16(void* dst, const void* src, bool have) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(have ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async8(void* dst, const void* src, bool have) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(have ? 8 : 0)
+               : "memory");
+}
+// Rows of a block of complex columns, row q from `src(q)`, `cols` of 32 columns.
+template <int ROWS, typename Src>
+__device__ __forceinline__ void fetch_columns(float2 (*dst)[32], Src src, int cols, bool wide) {
+  if (wide) {
+#pragma unroll
+    for (int e = threadIdx.x; e < ROWS * 16; e += kRowsThreads) {
+      const int q = e / 16, c = e % 16 * 2;
+      const float2* from = src(q);
+      copy_async16(&dst[q][c], c < cols ? from + c : from, c < cols);
+    }
+  } else {
+#pragma unroll 4
+    for (int e = threadIdx.x; e < ROWS * 32; e += kRowsThreads) {
+      const int q = e / 32, c = e % 32;
+      const float2* from = src(q);
+      copy_async8(&dst[q][c], c < cols ? from + c : from, c < cols);
+    }
+  }
+}
+// acc (rows x two columns) += a x, a = (ar, ai).
+template <int ROWS>
+__device__ __forceinline__ void rank1(float2 (&acc)[ROWS][2], const float (&ar)[ROWS],
+                                      const float (&ai)[ROWS], float4 x) {
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    acc[i][0].x = fmaf(ar[i], x.x, acc[i][0].x);
+    acc[i][0].y = fmaf(ar[i], x.y, acc[i][0].y);
+    acc[i][1].x = fmaf(ar[i], x.z, acc[i][1].x);
+    acc[i][1].y = fmaf(ar[i], x.w, acc[i][1].y);
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    acc[i][0].x = fmaf(-ai[i], x.y, acc[i][0].x);
+    acc[i][0].y = fmaf(ai[i], x.x, acc[i][0].y);
+    acc[i][1].x = fmaf(-ai[i], x.w, acc[i][1].x);
+    acc[i][1].y = fmaf(ai[i], x.z, acc[i][1].y);
+  }
+}
+__device__ __forceinline__ float lane4(const float4& v, int i) {
+  return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
+}
+
+// blockIdx = (strip of 32 columns, block of 16 rows, pencil).
+template <int T, int OP>
+__global__ void __launch_bounds__(kRowsThreads) solve_diag_rows_kernel(
+    int k, int nrhs, int64_t n_pad, const int32_t* __restrict__ diag_slot, int64_t n_slots,
+    const float* __restrict__ factor, const int32_t* __restrict__ pivots, const float2* work,
+    float2* ytmp, int wide) {
+  constexpr bool kAdj = OP == kUinvH || OP == kLinvH;
+  constexpr bool kLower = OP == kLinv || OP == kUinvH;     // columns up to the row
+  constexpr bool kUnit = OP == kLinv || OP == kLinvH;
+  constexpr int K = T < 64 ? T : 64, R = 16;               // depth of a chunk, rows of a block
+  constexpr int AR = kAdj ? K : R, AC = kAdj ? R : K;      // the chunk as it lies in the tile
+  __shared__ __align__(16) float a[2][AR][AC + 4];
+  __shared__ __align__(16) float2 x[K][32];
+  __shared__ int rows[T];
+  const int p = blockIdx.z, c0 = blockIdx.x * 32, m0 = blockIdx.y * R, tid = threadIdx.x;
+  const int cols = min(32, nrhs - c0), tr = tid / 16 * 2, tc = tid % 16 * 2;
+  const float* D = factor + tile_base(p, n_slots, diag_slot[k], T);
+  const int32_t* pv = pivots + (size_t)p * n_pad + (size_t)k * T;
+  launch_dependents();
+  if (tid < T) rows[tid] = kUnit ? pv[tid] : tid;
+  // the chunk at k0 of the block's rows of op(D), the other triangle zero
+  constexpr int kWords = 2 * AR * AC / 4 / kRowsThreads;
+  float4 w[kWords];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int t = 0; t < kWords; ++t) {
+      const int e = tid + t * kRowsThreads, plane = e / (AR * AC / 4);
+      const int r = e / (AC / 4) % AR, c = e % (AC / 4) * 4;
+      w[t] = *reinterpret_cast<const float4*>(
+          D + plane * T * T + (size_t)(kAdj ? k0 + r : m0 + r) * T + (kAdj ? m0 + c : k0 + c));
+    }
+  };
+  load(0);
+  __syncthreads();  // rows[]
+  wait_for_previous();
+  const float2* X = work + ((size_t)p * n_pad + (size_t)k * T) * nrhs + c0;
+  float2 acc[2][2] = {};
+#pragma unroll
+  for (int k0 = 0; k0 < T; k0 += K) {
+    if (k0 > 0) {
+      load(k0);
+      __syncthreads();
+    }
+    fetch_columns<K>(
+        x, [&](int q) { return X + (size_t)(OP == kLinv ? rows[k0 + q] : k0 + q) * nrhs; }, cols,
+        wide);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int t = 0; t < kWords; ++t) {
+      const int e = tid + t * kRowsThreads, plane = e / (AR * AC / 4);
+      const int r = e / (AC / 4) % AR, c = e % (AC / 4) * 4;
+      float v[4] = {w[t].x, w[t].y, w[t].z, w[t].w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int row = kAdj ? m0 + c + h : m0 + r, q = kAdj ? k0 + r : k0 + c + h;
+        if (kLower ? q > row : q < row) v[h] = 0.0f;
+        if (kUnit && q == row) v[h] = plane == 0 ? 1.0f : 0.0f;
+        if (kAdj && plane == 1) v[h] = -v[h];
+      }
+      *reinterpret_cast<float4*>(&a[plane][r][c]) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int lo = kLower ? 0 : max(m0 - k0, 0), hi = kLower ? min(m0 + R - k0, K) : K;
+#pragma unroll 2
+    for (int q = lo; q < hi; q += 4) {
+      float4 pr[2], pi[2];
+      if (!kAdj) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          pr[i] = *reinterpret_cast<const float4*>(&a[0][kAdj ? 0 : tr + i][q]);
+          pi[i] = *reinterpret_cast<const float4*>(&a[1][kAdj ? 0 : tr + i][q]);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        float ar[2], ai[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          ar[i] = kAdj ? a[0][kAdj ? q + h : 0][tr + i] : lane4(pr[i], h);
+          ai[i] = kAdj ? a[1][kAdj ? q + h : 0][tr + i] : lane4(pi[i], h);
+        }
+        rank1<2>(acc, ar, ai, *reinterpret_cast<const float4*>(&x[q + h][tc]));
+      }
+    }
+    if (k0 + K < T) __syncthreads();
+  }
+  float2* Y = ytmp + (size_t)p * T * nrhs + c0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = m0 + tr + i;
+    float2* to = Y + (size_t)(OP == kLinvH ? rows[r] : r) * nrhs + tc;
+    if (tc < cols) {
+      if (wide) {
+        *reinterpret_cast<float4*>(to) =
+            make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
+      } else {
+        to[0] = acc[i][0];
+        if (tc + 1 < cols) to[1] = acc[i][1];
+      }
+    }
+  }
+}
+
+// blockIdx.x = (tile of the list, block of 32 rows, strip of 32 columns), then
+// kCopyBlocks blocks that copy Y into X_k; blockIdx.y = pencil.
+template <int T, int OP>
+__global__ void __launch_bounds__(kRowsThreads) solve_update_rows_kernel(
+    int k, int n_items, int nrhs, int64_t n_pad, const int32_t* __restrict__ tiles,
+    const int32_t* __restrict__ slots, int64_t n_slots, const float* __restrict__ factor,
+    float2* work, const float2* ytmp, int wide) {
+  constexpr int K = 32, R = 32, kChunks = T / K, kBuffers = kChunks < 2 ? 1 : 2;
+  // a chunk of the block as it lies in the tile: [row][k] or [k][row]
+  __shared__ __align__(16) float a[kBuffers][2][32][36];
+  __shared__ __align__(16) float2 y[kBuffers][K][32];
+  const int p = blockIdx.y, tid = threadIdx.x;
+  const int ncs = (nrhs + 31) / 32, work_blocks = n_items * (T / R) * ncs;
+  const float2* Y = ytmp + (size_t)p * T * nrhs;
+  launch_dependents();
+  if ((int)blockIdx.x >= work_blocks) {
+    wait_for_previous();
+    float2* Xk = work + ((size_t)p * n_pad + (size_t)k * T) * nrhs;
+    const int total = T * nrhs;
+    for (int e = (blockIdx.x - work_blocks) * kRowsThreads + tid; e < total;
+         e += kCopyBlocks * kRowsThreads)
+      Xk[e] = Y[e];
+    return;
+  }
+  const int item = blockIdx.x / ((T / R) * ncs), rem = blockIdx.x % ((T / R) * ncs);
+  const int m0 = rem / ncs * R, c0 = rem % ncs * 32, cols = min(32, nrhs - c0);
+  const int tr = tid / 16 * 4, tc = tid % 16 * 2;
+  const float* F = factor + tile_base(p, n_slots, slots[item], T);
+  auto fetch_tile = [&](int c) {
+#pragma unroll
+    for (int t = 0; t < 2 * 32 * 8 / kRowsThreads; ++t) {
+      const int e = tid + t * kRowsThreads, plane = e / 256, r = e / 8 % 32, w = e % 8 * 4;
+      copy_async16(&a[c % kBuffers][plane][r][w],
+                   F + plane * T * T + (size_t)(OP == kPlain ? m0 + r : c * K + r) * T +
+                       (OP == kPlain ? c * K + w : m0 + w),
+                   true);
+    }
+  };
+  auto fetch_y = [&](int c) {
+    fetch_columns<K>(
+        y[c % kBuffers], [&](int q) { return Y + (size_t)(c * K + q) * nrhs + c0; }, cols, wide);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch_tile(0);
+  if (kChunks > 1) fetch_tile(1);
+  float2* X = work + ((size_t)p * n_pad + (size_t)tiles[item] * T + m0 + tr) * nrhs + c0 + tc;
+  wait_for_previous();
+  fetch_y(0);
+  if (kChunks > 1) fetch_y(1);
+  float4 old[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2* from = X + (size_t)i * nrhs;
+    old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (wide) {
+      if (tc < cols) old[i] = *reinterpret_cast<const float4*>(from);
+    } else {
+      if (tc < cols) { old[i].x = from[0].x; old[i].y = from[0].y; }
+      if (tc + 1 < cols) { old[i].z = from[1].x; old[i].w = from[1].y; }
+    }
+  }
+  float2 acc[4][2] = {};
+#pragma unroll 1
+  for (int c = 0; c < kChunks; ++c) {
+    if (c + 1 < kChunks)
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int b = c % kBuffers;
+#pragma unroll 4
+    for (int q = 0; q < K; q += 4) {
+      float4 pr[4], pi[4];  // plain: row tr + i, k q ..; conjugate: k q + i, rows tr ..
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        pr[i] = *reinterpret_cast<const float4*>(
+            OP == kPlain ? &a[b][0][tr + i][q] : &a[b][0][q + i][tr]);
+        pi[i] = *reinterpret_cast<const float4*>(
+            OP == kPlain ? &a[b][1][tr + i][q] : &a[b][1][q + i][tr]);
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        float ar[4], ai[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          ar[i] = OP == kPlain ? lane4(pr[i], h) : lane4(pr[h], i);
+          ai[i] = OP == kPlain ? lane4(pi[i], h) : -lane4(pi[h], i);
+        }
+        rank1<4>(acc, ar, ai, *reinterpret_cast<const float4*>(&y[b][q + h][tc]));
+      }
+    }
+    if (c + 2 < kChunks) {
+      __syncthreads();
+      fetch_tile(c + 2);
+      fetch_y(c + 2);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2* to = X + (size_t)i * nrhs;
+    const float4 v = make_float4(old[i].x - acc[i][0].x, old[i].y - acc[i][0].y,
+                                 old[i].z - acc[i][1].x, old[i].w - acc[i][1].y);
+    if (wide) {
+      if (tc < cols) *reinterpret_cast<float4*>(to) = v;
+    } else {
+      if (tc < cols) to[0] = make_float2(v.x, v.y);
+      if (tc + 1 < cols) to[1] = make_float2(v.z, v.w);
+    }
+  }
+}
+
+// The FP32 solve as a chain of programmatic launches.
+template <int T>
+int run_rows(const aosb_plan* P, const aosb_solve_args_v1* a, float2* Y, char* err, size_t cap) {
+  cudaStream_t st = (cudaStream_t)a->stream;
+  const int np = a->n_pencils, L = a->n_rhs, ncs = (L + 31) / 32;
+  float2* W = (float2*)a->work;
+  const int wide = L % 2 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)Y & 15) == 0;
+  bool first = true;
+  auto launch = [&](auto kernel, dim3 grid, auto... args) -> int {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = first ? 0 : 1;
+    first = false;
+    count_launches(1);
+    AOSB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...), err, cap);
+    return 0;
+  };
+  using Diag = void (*)(int, int, int64_t, const int32_t*, int64_t, const float*, const int32_t*,
+                        const float2*, float2*, int);
+  using Update = void (*)(int, int, int, int64_t, const int32_t*, const int32_t*, int64_t,
+                          const float*, float2*, const float2*, int);
+  auto step = [&](int k, Diag diag, Update update, const std::vector<int32_t>& off,
+                  const int32_t* tiles, const int32_t* slots) -> int {
+    const int n = off[k + 1] - off[k];
+    const double tile_bytes = 2.0 * T * T * sizeof(float), x_bytes = 2.0 * T * L * sizeof(float2);
+    cudaEvent_t ev[2];
+    bool timed = timing_begin(st, ev);
+    if (int rc = launch(diag, dim3(ncs, T / 16, np), k, L, P->n_pad, P->d_diag_slot, P->n_slots,
+                        a->factor, a->pivots, W, Y, wide))
+      return rc;
+    // algorithmic: one triangular T x T tile times T x L per pencil
+    if (timed)
+      timing_end(kTimedSolveDiag, st, ev, 4.0 * T * T * L * np, np * (tile_bytes + x_bytes));
+    timed = timing_begin(st, ev);
+    if (int rc = launch(update, dim3((unsigned)(n * (T / 32) * ncs + kCopyBlocks), np), k, n, L,
+                        P->n_pad, tiles + off[k], slots + off[k], P->n_slots, a->factor, W, Y,
+                        wide))
+      return rc;
+    // n tiles times T x L per pencil; factor tiles read once, X tiles read and
+    // written
+    if (timed)
+      timing_end(kTimedSolveUpdate, st, ev, 8.0 * T * T * L * (double)n * np,
+                 (double)n * np * (tile_bytes + x_bytes));
+    return 0;
+  };
+  const bool adj = a->adjoint != 0;
+  const Diag fd = adj ? solve_diag_rows_kernel<T, kUinvH> : solve_diag_rows_kernel<T, kLinv>;
+  const Diag bd = adj ? solve_diag_rows_kernel<T, kLinvH> : solve_diag_rows_kernel<T, kUinv>;
+  const Update up = adj ? solve_update_rows_kernel<T, kConjT> : solve_update_rows_kernel<T, kPlain>;
+  const int nb = (int)P->nb;
+  for (int k = 0; k < nb; ++k)
+    if (int rc = adj ? step(k, fd, up, P->ur_off, P->d_ur_tile, P->d_ur_slot)
+                     : step(k, fd, up, P->lb_off, P->d_lb_tile, P->d_lb_slot))
+      return rc;
+  for (int k = nb - 1; k >= 0; --k)
+    if (int rc = adj ? step(k, bd, up, P->ll_off, P->d_ll_tile, P->d_ll_slot)
+                     : step(k, bd, up, P->ua_off, P->d_ua_tile, P->d_ua_slot))
+      return rc;
+  return launch_check(err, cap, "solve");
+}
+
 template <int T>
 int run_solve(const aosb_plan* P, const aosb_solve_args_v1* a, char* err, size_t cap) {
   cudaStream_t st = (cudaStream_t)a->stream;
@@ -280,6 +638,9 @@ int run_solve(const aosb_plan* P, const aosb_solve_args_v1* a, char* err, size_t
       timing_end(kTimedSolveDiag, s, ev, 4.0 * T * T * L * np,
                  (double)np * (2.0 * T * T * sizeof(float) + 2.0 * T * L * sizeof(float2)));
   };
+  // factor storage that starts on no 16-byte boundary keeps the word-wise
+  // kernels below, which the tensor-core path without clusters shares
+  if (!tc && ((uintptr_t)a->factor & 15) == 0) return run_rows<T>(P, a, sl.y[0], err, cap);
   if (tc) AOSB_CUDA_TRY(cudaMemsetAsync(tc_status, 0, (size_t)np * sizeof(int32_t), st), err, cap);
   if (tc) {
     int rc = 0;
