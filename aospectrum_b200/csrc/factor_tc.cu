@@ -637,9 +637,7 @@ size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils) {
          kClaimBytes;
 }
 
-// Side stream of a caller stream for the lookahead panels (created once,
-// non-blocking, kept for the life of the process).
-static int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap) {
+int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap) {
   static std::mutex mu;
   static std::vector<std::pair<cudaStream_t, cudaStream_t>> table;
   int device = 0;
@@ -655,7 +653,9 @@ static int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t c
     }
   }
   cudaStream_t s = nullptr;
-  AOSB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), err, cap);
+  int least = 0, greatest = 0;
+  AOSB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest), err, cap);
+  AOSB_CUDA_TRY(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest), err, cap);
   table.emplace_back(main, s);
   *out = s;
   return 0;
