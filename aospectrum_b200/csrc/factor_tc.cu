@@ -7,12 +7,15 @@
 // update A_ij -= L_ik U_kj of every step run on the 5th generation tensor
 // cores:
 //
-//   * stage_kernel converts the step's L tiles (i,k) and U tiles (k,j) into
-//     four BF16 planes each -- re_hi, re_lo, im_hi, im_lo with
-//     x = hi + lo, hi = bf16(x), lo = bf16(x - hi) -- laid out as UMMA
-//     K-major, no-swizzle core matrices (8 rows x 16 bytes), cut into 16-wide
-//     K slabs so that one slab of one tile is a single contiguous bulk copy.
-//     For U the operand rows are U's columns (B is K-major).
+//   * Operands are staged as four BF16 planes each -- re_hi, re_lo, im_hi,
+//     im_lo with x = hi + lo, hi = bf16(x), lo = bf16(x - hi) -- laid out as
+//     UMMA K-major, no-swizzle core matrices (8 rows x 16 bytes), cut into
+//     16-wide K slabs so that one slab of one tile is a single contiguous bulk
+//     copy.  For U the operand rows are U's columns (B is K-major).
+//     stage_kernel converts the panel products' operands; their results L_ik
+//     and U_kj are written in this form by the panels' own epilogue, beside the
+//     FP32 tiles (a separate pass read every tile again: 32 pencils of 102
+//     steps 242 ms a factorization with it, 233 without, 1 pencil 17.3 / 16.7).
 //   * schur_tc_kernel: persistent and warp specialized (see the kernel).  Per
 //     16-wide K slab the MMA warp issues 12 tcgen05.mma.kind::f16 (M=N=128)
 //     into two FP32 TMEM accumulators:
@@ -83,6 +86,31 @@ __device__ __forceinline__ uint32_t pack_bf16x2(__nv_bfloat16 lo, __nv_bfloat16 
   return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
+// Eight consecutive k of one operand row, split, into a staged tile.
+__device__ __forceinline__ void store_chunk(unsigned char* out, int row, int k0,
+                                            const float (&re)[8], const float (&im)[8]) {
+  uint32_t plane[4][4];
+#pragma unroll
+  for (int t = 0; t < 8; t += 2) {
+    __nv_bfloat16 h[4][2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const __nv_bfloat16 rh = __float2bfloat16_rn(re[t + u]);
+      const __nv_bfloat16 ih = __float2bfloat16_rn(im[t + u]);
+      h[0][u] = rh;
+      h[1][u] = __float2bfloat16_rn(re[t + u] - __bfloat162float(rh));
+      h[2][u] = ih;
+      h[3][u] = __float2bfloat16_rn(im[t + u] - __bfloat162float(ih));
+    }
+#pragma unroll
+    for (int pl = 0; pl < 4; ++pl) plane[pl][t / 2] = pack_bf16x2(h[pl][0], h[pl][1]);
+  }
+#pragma unroll
+  for (int pl = 0; pl < 4; ++pl)
+    *reinterpret_cast<uint4*>(out + staged_offset(row, k0, pl)) =
+        make_uint4(plane[pl][0], plane[pl][1], plane[pl][2], plane[pl][3]);
+}
+
 __device__ __forceinline__ void stage_tile(const float* __restrict__ F, unsigned char* __restrict__ out,
                                            int kind, const int32_t* __restrict__ pv) {
   const bool a_side = kind == kStageA || kind == kStageAUnitLower;
@@ -127,26 +155,7 @@ __device__ __forceinline__ void stage_tile(const float* __restrict__ F, unsigned
           if (k0 + t > row) re[t] = im[t] = 0.0f;
       }
     }
-    uint32_t plane[4][4];
-#pragma unroll
-    for (int t = 0; t < 8; t += 2) {
-      __nv_bfloat16 h[4][2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const __nv_bfloat16 rh = __float2bfloat16_rn(re[t + u]);
-        const __nv_bfloat16 ih = __float2bfloat16_rn(im[t + u]);
-        h[0][u] = rh;
-        h[1][u] = __float2bfloat16_rn(re[t + u] - __bfloat162float(rh));
-        h[2][u] = ih;
-        h[3][u] = __float2bfloat16_rn(im[t + u] - __bfloat162float(ih));
-      }
-#pragma unroll
-      for (int pl = 0; pl < 4; ++pl) plane[pl][t / 2] = pack_bf16x2(h[pl][0], h[pl][1]);
-    }
-#pragma unroll
-    for (int pl = 0; pl < 4; ++pl)
-      *reinterpret_cast<uint4*>(out + staged_offset(row, k0, pl)) =
-          make_uint4(plane[pl][0], plane[pl][1], plane[pl][2], plane[pl][3]);
+    store_chunk(out, row, k0, re, im);
   }
 }
 
@@ -330,11 +339,15 @@ __device__ __forceinline__ int item_target(const ItemMap& m, int pair) {
   return m.tslot[a * m.nU + b];
 }
 
+// PANEL: the items are panel products, stored instead of added, and written a
+// second time as the Schur updates' operands.
+template <bool PANEL>
 __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
     const ItemMap map, int n_pencils, int64_t n_slots, const unsigned char* __restrict__ staging,
     int64_t staging_step_stride, int64_t staging_pencil_stride,
     int32_t* __restrict__ status, int* __restrict__ claim,
-    const __grid_constant__ CUtensorMap tmap_c, long long wl) {
+    const __grid_constant__ CUtensorMap tmap_c, long long wl,
+    unsigned char* staged_out) {
   const int n_pairs = map.n_pairs;
   extern __shared__ unsigned char dyn[];
   PShared& sh = *reinterpret_cast<PShared*>(
@@ -520,7 +533,7 @@ __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
     float* bre = sh.ep[warp][0];
     float* bim = sh.ep[warp][1];
     const int sw = lane & 7;
-    const bool store = map.kind == kMapPanel;
+    constexpr bool store = PANEL;
     const float sgn = store ? 1.0f : -1.0f;  // store acc / add -acc
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -582,6 +595,37 @@ __global__ void __launch_bounds__(kPThreads, 1) schur_tc_kernel(
             tma_reduce_add_2d(&tmap_c, bim, x, y + kTcT);
           }
           bulk_commit();
+        }
+        if (PANEL) {
+          // panels: the block as Schur operand, in place of the panel's own
+          unsigned char* tile = staged_out + (size_t)p * staging_pencil_stride +
+                                (size_t)pair * kStagedTileBytes;
+          const int n0 = half * 64 + bk * 32;
+          if (pair < map.nL) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              float xr[8], xi[8];
+#pragma unroll
+              for (int t = 0; t < 8; ++t) {
+                xr[t] = vr[c / 2][c % 2 * 8 + t];
+                xi[t] = vi[c / 2][c % 2 * 8 + t];
+              }
+              store_chunk(tile, quarter * 32 + lane, n0 + c * 8, xr, xi);
+            }
+          } else {
+            // columns of the block are operand rows: through its shared copy
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              float xr[8], xi[8];
+#pragma unroll
+              for (int t = 0; t < 8; ++t) {
+                const int off = (c * 8 + t) * 32 + (((lane >> 2) ^ t) << 2) + (lane & 3);
+                xr[t] = bre[off];
+                xi[t] = bim[off];
+              }
+              store_chunk(tile, n0 + lane, quarter * 32 + c * 8, xr, xi);
+            }
+          }
         }
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -696,8 +740,11 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   static std::atomic<uint64_t> attr_devices{0};
   const uint64_t dev_bit = device < 64 ? (uint64_t)1 << device : 0;
   if (dev_bit == 0 || (attr_devices.load() & dev_bit) == 0) {
-    cudaError_t e = cudaFuncSetAttribute(schur_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(
+        schur_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(schur_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem);
     if (e != cudaSuccess)
       return set_error(err, cap, AOSB_ERR_CUDA, "schur_tc smem attribute: %s", cudaGetErrorString(e));
     attr_devices.fetch_or(dev_bit);
@@ -762,12 +809,13 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
         nL, nU, 1, (int)k, lslot, uslot, P->diag_slot[k], P->n_slots, P->n_pad, a->factor,
         a->pivots, stage_buf(k), pencil_stride);
     const ItemMap pm{kMapPanel, nL, nU, nL + nU, 0, 0, 1, nullptr, lslot, uslot, nullptr};
-    schur_tc_kernel<<<grid_for((int64_t)(nL + nU) * np, cap_ctas), kPThreads, smem, s>>>(
-        pm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl);
+    schur_tc_kernel<true><<<grid_for((int64_t)(nL + nU) * np, cap_ctas), kPThreads, smem, s>>>(
+        pm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c,
+        wl, stage_buf(k));
     count_launches(2);
     return 0;
   };
-  // Schur staging of step k (L_ik as A, U_kj as B) on stream s
+  // Schur staging of step k (L_ik as A, U_kj as B) after FP32 panels, on stream s
   auto stage_schur = [&](int64_t k, cudaStream_t s) {
     const int nL = P->lb_off[k + 1] - P->lb_off[k];
     const int nU = P->ur_off[k + 1] - P->ur_off[k];
@@ -785,8 +833,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     const int nU = P->ur_off[k + 1] - P->ur_off[k];
     const ItemMap sm{kind, nL, nU, n_pairs, a0, b0, 1, P->d_sc_slot + P->sc_off[k], nullptr, nullptr,
                      nullptr};
-    schur_tc_kernel<<<grid_for((int64_t)n_pairs * np, cap_ctas), kPThreads, smem, s>>>(
-        sm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl);
+    schur_tc_kernel<false><<<grid_for((int64_t)n_pairs * np, cap_ctas), kPThreads, smem, s>>>(
+        sm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl,
+        nullptr);
     count_launches(1);
   };
   // Schur update of step k (the pairs `kind` selects) on the caller stream,
@@ -799,8 +848,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     const bool timed = timing_begin(st, ev);
     const ItemMap sm{kind, nL, nU, n_pairs, a0, b0, 1, P->d_sc_slot + P->sc_off[k], nullptr, nullptr,
                      nullptr};
-    schur_tc_kernel<<<grid_for(items, cap_ctas), kPThreads, smem, st>>>(
-        sm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl);
+    schur_tc_kernel<false><<<grid_for(items, cap_ctas), kPThreads, smem, st>>>(
+        sm, np, P->n_slots, stage_buf(k), buffer_bytes, pencil_stride, a->status, nullptr, tmap_c, wl,
+        nullptr);
     count_launches(1);
     if (timed)
       timing_end(kTimedSchur, st, ev, (double)items * 8.0 * kTcT * kTcT * kTcT,
@@ -851,9 +901,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
       if (rc != 0 && pair_rc == 0) pair_rc = rc;
     } else {
       const ItemMap lm{kMapList, 0, 0, (int)n, 0, 0, 2, nullptr, nullptr, nullptr, dev + 5 * off[ss]};
-      schur_tc_kernel<<<grid_for(n * np, cap_ctas), kPThreads, smem, s>>>(
+      schur_tc_kernel<false><<<grid_for(n * np, cap_ctas), kPThreads, smem, s>>>(
           lm, np, P->n_slots, stage_buf(k0), buffer_bytes, pencil_stride, a->status, claim,
-          tmap_c, wl);
+          tmap_c, wl, nullptr);
       count_launches(1);
     }
     // algorithmic bytes: every target read and written once, the staged L
@@ -888,8 +938,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     const bool timed = count_work && timing_begin(s, ev);
     const ItemMap lm{kMapList, 0, 0, (int)n, 0, 0, kMaxSteps, nullptr, nullptr, nullptr,
                      P->d_qs_items + (1 + 2 * kMaxSteps) * i0};
-    schur_tc_kernel<<<grid_for(n * np, cap_ctas), kPThreads, smem, s>>>(
-        lm, np, P->n_slots, stage_buf(k0), buffer_bytes, pencil_stride, a->status, claim, tmap_c, wl);
+    schur_tc_kernel<false><<<grid_for(n * np, cap_ctas), kPThreads, smem, s>>>(
+        lm, np, P->n_slots, stage_buf(k0), buffer_bytes, pencil_stride, a->status, claim, tmap_c, wl,
+        nullptr);
     count_launches(1);
     if (timed) {
       double products = 0;
@@ -920,7 +971,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
                           P->schur_updates * np >= 10000 * P->nb;
   if (four_steps) {
     const int64_t nb = P->nb;
-    // the group's panels and staging, each after the updates of the group's
+    // the group's panels, each after the updates of the group's
     // earlier steps to that step's tile row and column
     auto prepare = [&](int64_t g, cudaStream_t s, int cap_ctas) -> int {
       for (int m = 0; m < kMaxSteps; ++m) {
@@ -928,7 +979,6 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
         if (k >= nb) break;
         if (m > 0) four_step(g, m - 1, cap_ctas, s, nullptr, false);
         if (int rc = panels(k, s, cap_ctas)) return rc;
-        stage_schur(k, s);
       }
       return 0;
     };
@@ -949,11 +999,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   if (two_steps) {
     const int64_t nb = P->nb;
     if (int rc = panels(0, st, sms)) return rc;
-    stage_schur(0, st);
     if (nb > 1) {
       inner(0, st, sms);
       if (int rc = panels(1, st, sms)) return rc;
-      stage_schur(1, st);
     }
     for (int64_t ss = 0; 2 * ss + 1 < nb; ++ss) {
       const int64_t k2 = 2 * ss + 2, k3 = 2 * ss + 3;
@@ -966,11 +1014,9 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
         AOSB_CUDA_TRY(cudaEventRecord(ev_cross, st), err, cap);
         AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_cross, 0), err, cap);
         if (int rc = panels(k2, side, reserve)) return rc;
-        stage_schur(k2, side);
         if (k3 < nb) {
           inner(k2, side, reserve);
           if (int rc = panels(k3, side, reserve)) return rc;
-          stage_schur(k3, side);
         }
         // main launch first: it starts at once either way, and a profiler
         // that serializes launches then sees the full-grid launch take the
@@ -1001,13 +1047,11 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     }
     if (k == 0) {
       if (int rc = panels(0, st, sms)) return rc;
-      stage_schur(0, st);
     }
     const bool has_next = k + 1 < P->nb;
     if (nL == 0 || nU == 0) {
       if (has_next) {
         if (int rc = panels(k + 1, st, sms)) return rc;
-        stage_schur(k + 1, st);
       }
       continue;
     }
@@ -1015,7 +1059,6 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
       schur(k, kMapSchur, 0, 0, nL * nU, sms);
       if (has_next) {
         if (int rc = panels(k + 1, st, sms)) return rc;
-        stage_schur(k + 1, st);
       }
       continue;
     }
@@ -1027,7 +1070,6 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     AOSB_CUDA_TRY(cudaEventRecord(ev_cross, st), err, cap);
     AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_cross, 0), err, cap);
     if (int rc = panels(k + 1, side, reserve)) return rc;
-    stage_schur(k + 1, side);
     AOSB_CUDA_TRY(cudaEventRecord(ev_panel, side), err, cap);
     if (rest > 0) schur(k, kMapRest, a0, b0, rest, sms - reserve);
     AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev_panel, 0), err, cap);
