@@ -225,7 +225,10 @@ int aospectrum_b200_solve_complex64_ubatch_v1(const aospectrum_b200_ubatch_reque
     cudaFree(d_work); cudaFree(d_factor); cudaFree(d_piv); cudaFree(d_status); cudaFree(d_pk);
     cudaFree(d_shift);
     cudaFree(d_solve_scratch);
-    if (st) cudaStreamDestroy(st);
+    if (st) {
+      side_stream_forget(st);
+      cudaStreamDestroy(st);
+    }
   };
   auto cuda_ok = [&](cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;

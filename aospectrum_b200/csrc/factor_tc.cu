@@ -681,13 +681,16 @@ size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils) {
          kClaimBytes;
 }
 
+namespace {
+std::mutex g_side_mutex;
+std::vector<std::pair<cudaStream_t, cudaStream_t>> g_side_streams;  // (caller's, side)
+}  // namespace
+
 int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap) {
-  static std::mutex mu;
-  static std::vector<std::pair<cudaStream_t, cudaStream_t>> table;
   int device = 0;
   cudaGetDevice(&device);
-  std::lock_guard<std::mutex> lock(mu);
-  for (auto& e : table) {
+  std::lock_guard<std::mutex> lock(g_side_mutex);
+  for (auto& e : g_side_streams) {
     if (e.first == main) {
       int dev2 = -1;
       if (cudaStreamGetDevice(e.second, &dev2) == cudaSuccess && dev2 == device) {
@@ -700,9 +703,18 @@ int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap) {
   int least = 0, greatest = 0;
   AOSB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest), err, cap);
   AOSB_CUDA_TRY(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest), err, cap);
-  table.emplace_back(main, s);
+  g_side_streams.emplace_back(main, s);
   *out = s;
   return 0;
+}
+
+void side_stream_forget(cudaStream_t main) {
+  std::lock_guard<std::mutex> lock(g_side_mutex);
+  for (size_t i = g_side_streams.size(); i-- > 0;) {
+    if (g_side_streams[i].first != main) continue;
+    cudaStreamDestroy(g_side_streams[i].second);
+    g_side_streams.erase(g_side_streams.begin() + (std::ptrdiff_t)i);
+  }
 }
 
 // Tensor map of the factor storage as a [rows][T] FP32 matrix (each tile is
