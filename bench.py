@@ -757,7 +757,9 @@ def main() -> None:
         peak = sustained if sustained else 1400.0
         achieved = k_flops.value / (k_ms.value / 1e3) / 1e12
         per_launch_units = k_flops.value / k_launches.value / (8.0 * info.tile ** 3)
-        traffic = schur_traffic_per_unit()
+        # c2 takes four steps at a time from 8 pencils on
+        traffic = schur_traffic_per_unit(
+            "four" if np.mean(eng.factor_pencils or [1]) >= 8 and not args.schur_pairs else "two")
         roofline = {
             "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak,
@@ -934,12 +936,12 @@ def main() -> None:
         dist.destroy_process_group()
 
 
-def schur_traffic_per_unit() -> dict | None:
+def schur_traffic_per_unit(steps: str) -> dict | None:
     """DRAM bytes per algorithmic unit of schur_tc_kernel -- one (target
     tile, tile step, pencil) update, 8 T^3 flops -- from the committed ncu
-    capture summary of the two-step kernel (dram__bytes_read.sum +
+    capture summary of the two- or four-step kernel (dram__bytes_read.sum +
     write.sum of the captured launch divided by the units it applied)."""
-    f = ROOT / "profiles" / "schur_tc_kernel_two_step_c2.json"
+    f = ROOT / "profiles" / f"schur_tc_kernel_{steps}_step_c2.json"
     if not f.exists():
         return None
     d = json.loads(f.read_text())
