@@ -362,8 +362,11 @@ int ensure_diag_attr(char* err, size_t cap) {
   const uint64_t dev_bit = device < 64 ? (uint64_t)1 << device : 0;
   if (dev_bit != 0 && (attr_devices.load() & dev_bit) != 0) return 0;
   const size_t diag_smem = diag_smem_bytes<T>();
-  cudaError_t e = cudaFuncSetAttribute(diag_lu_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)diag_smem);
+  cudaError_t e = cudaFuncSetAttribute(
+      diag_lu_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(diag_lu_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)diag_smem);
   if (e != cudaSuccess)
     return set_error(err, cap, AOSB_ERR_CUDA, "diag_lu smem attribute: %s", cudaGetErrorString(e));
   attr_devices.fetch_or(dev_bit);
@@ -373,8 +376,9 @@ int ensure_diag_attr(char* err, size_t cap) {
 // Diagonal LU of step k (FP32 SIMT) on stream st.
 template <int T>
 void step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int64_t k, cudaStream_t st,
-               float* diag_tiles = nullptr) {
-  diag_lu_kernel<T><<<a->n_pencils, DiagShape<T>::kThreads, diag_smem_bytes<T>(), st>>>(
+               bool real = false, float* diag_tiles = nullptr) {
+  const auto kernel = real ? diag_lu_kernel<T, true> : diag_lu_kernel<T, false>;
+  kernel<<<a->n_pencils, DiagShape<T>::kThreads, diag_smem_bytes<T>(), st>>>(
       (int)k, P->d_diag_slot, P->n_slots, P->n_pad, a->factor, a->pivots, a->status, diag_tiles);
   count_launches(1);
 }
@@ -413,7 +417,7 @@ int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
       if (done) cudaEventDestroy(done);
     }
   } ev;
-  step_diag<T>(P, a, 0, st, diag_tiles);
+  step_diag<T>(P, a, 0, st, real, diag_tiles);
   for (int64_t k = 0; k < P->nb; ++k) {
     step_panels<T>(P, a, k, real);
     const int nL = P->lb_off[k + 1] - P->lb_off[k];
@@ -422,7 +426,7 @@ int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     const bool next = k + 1 < P->nb;
     if (!next || targets * SchurCfg<T>::kSub * a->n_pencils < kLookaheadBlocks) {
       if (int rc = launch_schur<T>(P, a, k, nU, 0, targets, real, err, cap)) return rc;
-      if (next) step_diag<T>(P, a, k + 1, st, diag_tiles);
+      if (next) step_diag<T>(P, a, k + 1, st, real, diag_tiles);
       continue;
     }
     if (side == nullptr) {
@@ -436,7 +440,7 @@ int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     if (int rc = launch_schur<T>(P, a, k, nU, 0, head, real, err, cap)) return rc;
     AOSB_CUDA_TRY(cudaEventRecord(ev.ready, st), err, cap);
     AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev.ready, 0), err, cap);
-    step_diag<T>(P, a, k + 1, side, diag_tiles);
+    step_diag<T>(P, a, k + 1, side, real, diag_tiles);
     AOSB_CUDA_TRY(cudaEventRecord(ev.done, side), err, cap);
     if (int rc = launch_schur<T>(P, a, k, nU, head, targets - head, real, err, cap)) return rc;
     AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev.done, 0), err, cap);
@@ -487,7 +491,7 @@ int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cu
                      char* err, size_t cap) {
   if (P->T != 128) return set_error(err, cap, AOSB_ERR_UNSUPPORTED, "diagonal step needs tile 128");
   if (int rc = ensure_diag_attr<128>(err, cap)) return rc;
-  diag_lu_kernel<128><<<a->n_pencils, DiagShape<128>::kThreads, diag_smem_bytes<128>(), st>>>(
+  diag_lu_kernel<128, false><<<a->n_pencils, DiagShape<128>::kThreads, diag_smem_bytes<128>(), st>>>(
       k, P->d_diag_slot, P->n_slots, P->n_pad, a->factor, a->pivots, a->status, nullptr);
   count_launches(1);
   return 0;
