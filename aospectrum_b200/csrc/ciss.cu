@@ -258,6 +258,7 @@ __global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads
     for (int q = 0; q < kNormThreads / 8; ++q) t += part[q][threadIdx.x];
     sum[threadIdx.x] = t;
   }
+  __syncwarp();  // the aligned barrier wants the whole warp together
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                    : "memory");
   if (rank == 0 && threadIdx.x < 8 && j < m) {

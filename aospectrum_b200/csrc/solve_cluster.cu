@@ -154,6 +154,7 @@ __device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, lon
   return false;
 }
 __device__ __forceinline__ void cluster_meet() {
+  __syncwarp();  // the aligned forms want the whole warp together
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                    : "memory");
 }
