@@ -642,7 +642,7 @@ int run_solve(const aosb_plan* P, const aosb_solve_args_v1* a, char* err, size_t
   // kernels below, which the tensor-core path without clusters shares
   if (!tc && ((uintptr_t)a->factor & 15) == 0) return run_rows<T>(P, a, sl.y[0], err, cap);
   if (tc) AOSB_CUDA_TRY(cudaMemsetAsync(tc_status, 0, (size_t)np * sizeof(int32_t), st), err, cap);
-  if (tc) {
+  if (tc && (a->flags & AOSB_SOLVE_PER_STEP) == 0) {
     int rc = 0;
     cudaEvent_t ev[2];
     const bool timed = timing_begin(st, ev);

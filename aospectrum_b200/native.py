@@ -27,6 +27,7 @@ PRECISION_BF16X3_FP32_PANELS = 2
 PRECISION_BF16X3_ONE_STEP = 3
 SOLVE_TENSOR_CORES = 1
 SOLVE_GRAPH = 2
+SOLVE_PER_STEP = 4
 
 STATUS_NAMES = {
     10: "ABI mismatch", 11: "dimensions", 12: "batch", 13: "null pointer",

@@ -366,6 +366,11 @@ int64_t aosb_tc_set_wait_limit(int64_t polls);
  * the stream is being captured by the caller.  Graphs are released with
  * their plan. */
 #define AOSB_SOLVE_GRAPH 2
+/* AOSB_SOLVE_PER_STEP: with AOSB_SOLVE_TENSOR_CORES, one launch per diagonal
+ * step and one per update whatever the batch (the form that
+ * aosb_solve_set_ctas_per_sm and aosb_solve_set_lookahead act on), so that a
+ * pencil's result does not depend on how many are solved with it. */
+#define AOSB_SOLVE_PER_STEP 4
 
 typedef struct {
   uint32_t abi_version;
