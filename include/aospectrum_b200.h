@@ -355,9 +355,14 @@ int64_t aosb_tc_set_wait_limit(int64_t polls);
  * updates on the tensor cores in split BF16 (FP32 accumulation); 0 keeps
  * them in FP32 SIMT.  The tensor-core updates bound their waits; after the
  * solves, aosb_solve_check synchronizes the stream and reports a timeout.
- * Up to some 70 units (pencils x strips of 32 right-hand sides) the sweeps run
- * as one launch of thread-block clusters, past that as one launch per diagonal
- * step and one per update; the two forms round differently.
+ * Tensor-core sweeps run as one launch of thread-block clusters or as one launch
+ * per diagonal step and one per update, whichever is estimated to be faster for
+ * the plan's tiles a step, the units (pencils x strips of 32 right-hand sides)
+ * and the columns of a strip: clusters for nearly all batches of up to about 74
+ * units and for any number on plans of few tiles, and otherwise by the size of
+ * the last wave of clusters.  The two forms round differently, so a pencil's
+ * result can depend on the batch it is solved in; AOSB_SOLVE_PER_STEP fixes the
+ * form.
  * ------------------------------------------------------------------------ */
 #define AOSB_SOLVE_TENSOR_CORES 1
 /* AOSB_SOLVE_GRAPH: capture the solve's launch sequence into a CUDA graph

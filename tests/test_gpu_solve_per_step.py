@@ -75,3 +75,29 @@ def test_variants_agree(case, adjoint, columns):
         for p in range(len(shifts)):
             err = np.linalg.norm(one[p] - other[p]) / np.linalg.norm(other[p])
             assert err < 1e-3, (p, err)
+
+
+def test_the_rule_gives_a_large_batch_to_this_form():
+    """108 units on 75 steps, where it is 7 % ahead of the clusters: 18 pencils,
+    six strips of which the last one is ragged."""
+    import torch
+
+    from aospectrum_b200 import native, synth
+
+    torch.cuda.set_device(0)
+    b = synth.generate_bundle(replace(synth.SPEC_C2, name="cubic9", grid=(9, 9, 9),
+                                      cell=(21.6, 21.6, 21.6), seed=17))
+    dev, plan, h, s = _pencil_case(b, bundles.KPOINTS[2], torch, 128, "natural")
+    try:
+        assert plan.info.n_tiles == 75
+        rng = np.random.default_rng(5)
+        rhs = rng.standard_normal((dev.n, 190)) + 1j * rng.standard_normal((dev.n, 190))
+        shifts = np.linspace(-2.6, 0.5, 18) + 0.3j
+        auto, steps = (_factor_solve(dev, plan, h, s, shifts, rhs, torch, flags=flags,
+                                     precision=native.PRECISION_BF16X3)
+                       for flags in (native.SOLVE_TENSOR_CORES,
+                                     native.SOLVE_TENSOR_CORES | native.SOLVE_PER_STEP))
+        assert np.array_equal(auto, steps)
+    finally:
+        dev.close()
+        plan.close()
