@@ -181,33 +181,51 @@ def hermitize(a: np.ndarray) -> np.ndarray:
 class _SmallLapack:
     """Host LAPACK on one thread while any thread is inside.  The library
     handles are looked up once (finding them walks every loaded library, which
-    takes longer than the eigenproblems), and the first thread in and the last
-    one out change the limit, so overlapping users cannot restore each other's."""
+    takes longer than the eigenproblems).  A BLAS pool's limit is the
+    process's, so the first thread in and the last one out change it and
+    overlapping users cannot restore each other's; an OpenMP limit is its
+    thread's own, so each thread sets and restores that for itself."""
 
     def __init__(self) -> None:
         self._lock = threading.Lock()
-        self._controller: Any = None
+        self._libraries: dict[str, list[Any]] | None = None
         self._inside = 0
-        self._limit: Any = None
+        self._blas: list[int | None] = []
+        self._mine = threading.local()
+
+    def _limit(self, api: str) -> list[int | None]:
+        """One thread for the libraries of an API; the counts they had (None
+        where a library does not tell)."""
+        before = [lib.get_num_threads() for lib in self._libraries[api]]
+        self._set(api, [1] * len(before))
+        return before
+
+    def _set(self, api: str, counts: list[int | None]) -> None:
+        for lib, count in zip(self._libraries[api], counts):
+            if count is not None:
+                lib.set_num_threads(count)
 
     def __enter__(self) -> None:
         with self._lock:
-            if self._inside == 0:
-                if self._controller is None:
-                    from scipy import linalg  # noqa: F401  (loads its own BLAS)
-                    from threadpoolctl import ThreadpoolController
+            if self._libraries is None:
+                from scipy import linalg  # noqa: F401  (loads its own BLAS)
+                from threadpoolctl import ThreadpoolController
 
-                    self._controller = ThreadpoolController()
-                self._limit = self._controller.limit(limits=1)
-                self._limit.__enter__()
+                found = ThreadpoolController().lib_controllers
+                self._libraries = {api: [lib for lib in found if lib.user_api == api]
+                                   for api in ("blas", "openmp")}
+            openmp = self._limit("openmp")
+            if self._inside == 0:
+                self._blas = self._limit("blas")
             self._inside += 1
+        self._mine.__dict__.setdefault("openmp", []).append(openmp)
 
     def __exit__(self, *exc: Any) -> None:
         with self._lock:
             self._inside -= 1
             if self._inside == 0:
-                limit, self._limit = self._limit, None
-                limit.__exit__(*exc)
+                self._set("blas", self._blas)
+            self._set("openmp", self._mine.openmp.pop())
 
 
 _SMALL_LAPACK = _SmallLapack()
