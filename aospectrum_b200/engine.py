@@ -22,6 +22,7 @@ of the reference (``src/aospectrum/sparse.py:199-245``,
 
 from __future__ import annotations
 
+import contextlib
 import math
 import os
 from concurrent.futures import ThreadPoolExecutor
@@ -728,12 +729,20 @@ class BandEngine:
                         self.pattern.nnz, pk.data_ptr(), z.contiguous().data_ptr(),
                         b.data_ptr(), n * L, xn.data_ptr(), rr.data_ptr(), st)
 
-    def _host_map(self, fn, items: list) -> list:
-        """fn over items: the small FP64 eigenproblems of the batch's k points
-        run in parallel threads, each on one BLAS thread (numpy and scipy
-        release the GIL inside LAPACK)."""
+    # Widest projected problem of a single k point that runs on one BLAS thread.
+    # Between stages of GPU work a pool of 16 threads costs 40-150 ms a call to
+    # wake, so it pays only where one thread takes longer than that.  ms a call,
+    # one thread / the pool, 3328 orbitals: 128 wide 12.4 / 122, 256: 24.6 / 96,
+    # 384: 53 / 140, 512: 126 / 154, 1024: 922 / 354.
+    one_thread_width = 512
+
+    def _host_map(self, fn, items: list, width: int = 0) -> list:
+        """fn over items: the small FP64 eigenproblems (at most ``width`` wide)
+        of the batch's k points run in parallel threads, each on one BLAS thread
+        (numpy and scipy release the GIL inside LAPACK); a single wide one gets
+        the BLAS pool."""
         if len(items) <= 1:
-            with small_lapack():
+            with small_lapack() if width <= self.one_thread_width else contextlib.nullcontext():
                 return [fn(x) for x in items]
         if self._lapack_pool is None:
             self._lapack_pool = ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1))
@@ -760,7 +769,8 @@ class BandEngine:
             grams.append(self._gram(mom[k], sm))
         grams = torch.stack(grams).cpu().numpy()
         tol = st.rank_relative_tolerance
-        trunc = self._host_map(lambda g: truncate_gram(g, tol, limit_threads=False), list(grams))
+        trunc = self._host_map(lambda g: truncate_gram(g, tol, limit_threads=False), list(grams),
+                               grams.shape[-1])
         basis = [self._dense_mul(mom[k], torch.from_numpy(trunc[k][0]).to(dev)) for k in range(nk)]
         torch.cuda.current_stream(dev).synchronize()
         dt = (perf_counter() - t) / nk
@@ -776,7 +786,8 @@ class BandEngine:
             self._spmm(svals[k], basis[k], sb)
             pairs.append((self._gram(basis[k], hb), self._gram(basis[k], sb)))
         pairs = [(hr.cpu().numpy(), sr.cpu().numpy()) for hr, sr in pairs]
-        eig = self._host_map(lambda p: projected_eigh(p[0], p[1], limit_threads=False), pairs)
+        eig = self._host_map(lambda p: projected_eigh(p[0], p[1], limit_threads=False), pairs,
+                             max((hr.shape[0] for hr, _ in pairs), default=0))
         dt = (perf_counter() - t) / nk
         for d in local:
             d["rayleigh_ritz"] = dt

@@ -10,6 +10,7 @@ import threading
 
 import numpy as np
 import scipy.linalg  # noqa: F401  (loads its own BLAS)
+import pytest
 from threadpoolctl import threadpool_info, threadpool_limits
 
 
@@ -97,3 +98,18 @@ def test_nested_use_restores_the_limits():
         assert set(_threads("blas").values()) == {1}
         assert set(_threads("openmp").values()) <= {1}
     assert (_threads("blas"), _threads("openmp")) == before
+
+
+@pytest.mark.parametrize("width,items,one", [(0, 1, True), (512, 1, True), (513, 1, False),
+                                             (1024, 1, False), (1024, 2, True)])
+def test_a_single_wide_problem_keeps_the_blas_pool(width, items, one):
+    from aospectrum_b200.engine import BandEngine
+
+    eng = BandEngine.__new__(BandEngine)   # host part only: no device state
+    eng._lapack_pool = None
+    with threadpool_limits(limits=4, user_api="blas"):
+        pool = _threads("blas")
+        got = eng._host_map(lambda _: _threads("blas"), list(range(items)), width)
+    assert got == [dict.fromkeys(pool, 1) if one else pool] * items
+    if eng._lapack_pool is not None:
+        eng._lapack_pool.shutdown()
