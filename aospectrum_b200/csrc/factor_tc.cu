@@ -671,13 +671,16 @@ static int64_t staged_tiles_per_pencil(const aosb_plan* P) {
 
 // Staging buffers: the steps of two groups, since the next group is staged
 // while the update of the current one still reads its own -- four with
-// two-step updates, eight where the plan has four-step lists.  After them,
-// 256 bytes hold the item counter of the shared updates.
-static int stage_buffers(const aosb_plan* P) { return P->qs_items.empty() ? 4 : 2 * kMaxSteps; }
+// two-step updates, eight for batches that are updated four steps at a time.
+// After them, 256 bytes hold the item counter of the shared updates.  The count
+// does not fall with the batch, so the workspace of a batch serves smaller ones.
+static int stage_buffers(const aosb_plan* P, int32_t n_pencils) {
+  return four_steps_for(P, n_pencils) ? 2 * kMaxSteps : 4;
+}
 constexpr size_t kClaimBytes = 256;
 size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils) {
   if (P->T != kTcT) return 0;
-  return stage_buffers(P) * (size_t)staged_tiles_per_pencil(P) * kStagedTileBytes * (size_t)n_pencils +
+  return stage_buffers(P, n_pencils) * (size_t)staged_tiles_per_pencil(P) * kStagedTileBytes * (size_t)n_pencils +
          kClaimBytes;
 }
 
@@ -805,7 +808,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     }
   } guard{ev_cross, ev_panel};
   const int64_t buffer_bytes = (int64_t)np * pencil_stride;
-  const int n_buffers = stage_buffers(P);
+  const int n_buffers = stage_buffers(P, np);
   auto stage_buf = [&](int64_t k) { return staging + (k % n_buffers) * buffer_bytes; };
 
   // diagonal LU + panel products of step k on stream s (panel grid <= cap_ctas)
@@ -938,7 +941,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   // k + 2, k + 3 go first; the side stream then prepares the next
   // super-step's two panels beside the rest.
   const bool two_steps = tc_panels && lookahead && a->precision == AOSB_PRECISION_BF16X3 &&
-                         P->d_ss_rest != nullptr;
+                         !P->ss_rest.empty();
   // Four-step (K <= 512) updates: the same scheme with groups of four steps.
   // List `l` (plan.h) of group g on stream s.
   auto four_step = [&](int64_t g, int l, int cap_ctas, cudaStream_t s, int* claim = nullptr,
@@ -955,10 +958,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
         nullptr);
     count_launches(1);
     if (timed) {
-      double products = 0;
-      for (int64_t i = i0; i < i1; ++i)
-        for (int h = 0; h < kMaxSteps; ++h)
-          products += P->qs_items[(1 + 2 * kMaxSteps) * i + 1 + 2 * h] >= 0 ? 1 : 0;
+      const double products = (double)P->qs_products[5 * g + l];
       const int64_t k1 = std::min<int64_t>(k0 + kMaxSteps, P->nb);
       const double staged =
           (double)(P->lb_off[k1] - P->lb_off[k0] + P->ur_off[k1] - P->ur_off[k0]);
@@ -979,8 +979,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   // 34.2, x 8: 66.7 / 63.1, x 32: 257 / 241; 951 x 8: 33.3 / 34.1, x 16: 65.8 /
   // 63.8, x 64: 260 / 246; 522 x 8: 16.0 / 17.0, x 24: 39.6 / 37.9; 3043 x 2:
   // 62.7 / 60.5, x 8: 230 / 216; 301 x 64: 45.8 / 46.3; 195 x 64: 103.8 / 111.4.
-  const bool four_steps = two_steps && !pairs && P->d_qs_items != nullptr &&
-                          P->schur_updates * np >= 10000 * P->nb;
+  const bool four_steps = two_steps && !pairs && four_steps_for(P, np);
   if (four_steps) {
     const int64_t nb = P->nb;
     // the group's panels, each after the updates of the group's

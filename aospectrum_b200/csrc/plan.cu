@@ -331,6 +331,12 @@ void build_super_steps(aosb_plan* P) {
   }
 }
 
+// The plan has four-step lists and this batch is long enough for them (why the
+// line lies there: factor_tc.cu).
+bool four_steps_for(const aosb_plan* P, int64_t n_pencils) {
+  return !P->qs_products.empty() && P->schur_updates * n_pencils >= 10000 * P->nb;
+}
+
 // Four-step Schur item lists (see plan.h).  The targets of a group are
 // gathered row by row, so a group costs one pass over its (L, U) pairs.
 void build_quad_steps(aosb_plan* P) {
@@ -338,6 +344,7 @@ void build_quad_steps(aosb_plan* P) {
   const int64_t nb = P->nb;
   P->qs_off.assign(1, 0);
   P->qs_items.clear();
+  P->qs_products.clear();
   struct Item {
     int32_t j, e[2 * kSteps];
   };
@@ -382,6 +389,10 @@ void build_quad_steps(aosb_plan* P) {
       }
     }
     for (auto& l : lists) {
+      int64_t products = 0;
+      for (size_t i = 0; i < l.size(); i += 1 + 2 * kSteps)
+        for (int s = 0; s < kSteps; ++s) products += l[i + 1 + 2 * s] >= 0 ? 1 : 0;
+      P->qs_products.push_back(products);
       P->qs_items.insert(P->qs_items.end(), l.begin(), l.end());
       P->qs_off.push_back((int64_t)P->qs_items.size() / (1 + 2 * kSteps));
     }
@@ -677,8 +688,13 @@ int aosb_plan_upload(aosb_plan_t* P, char* err, size_t cap) {
   if (P->uploaded) return 0;
   int rc = aosb::plan_upload(P, err, cap);
   if (rc == 0) rc = aosb::up(&P->d_indptr, P->h_indptr, err, cap);
-  if (rc == 0 && !P->ss_cross.empty()) rc = aosb::up(&P->d_ss_cross, P->ss_cross, err, cap);
-  if (rc == 0 && !P->ss_rest.empty()) rc = aosb::up(&P->d_ss_rest, P->ss_rest, err, cap);
+  // Where four steps serve every batch, the two-step lists (10 bytes a tile
+  // product, as many as the four-step ones that take their place) stay on the
+  // host: only the two-CTA pairs run two steps then, from lists of their own.
+  const bool two = !aosb::four_steps_for(P, 1);
+  if (rc == 0 && two && !P->ss_cross.empty())
+    rc = aosb::up(&P->d_ss_cross, P->ss_cross, err, cap);
+  if (rc == 0 && two && !P->ss_rest.empty()) rc = aosb::up(&P->d_ss_rest, P->ss_rest, err, cap);
   if (rc == 0 && !P->sp_cross.empty()) rc = aosb::up(&P->d_sp_cross, P->sp_cross, err, cap);
   if (rc == 0 && !P->sp_rest.empty()) rc = aosb::up(&P->d_sp_rest, P->sp_rest, err, cap);
   if (rc == 0 && !P->qs_items.empty()) rc = aosb::up(&P->d_qs_items, P->qs_items, err, cap);
@@ -688,6 +704,7 @@ int aosb_plan_upload(aosb_plan_t* P, char* err, size_t cap) {
     return rc;
   }
   P->uploaded = true;
+  std::vector<int32_t>().swap(P->qs_items);  // only the device reads them from here on
   return 0;
 }
 

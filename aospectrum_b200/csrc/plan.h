@@ -47,8 +47,9 @@ struct aosb_plan {
   // q = 4g+4 .. 4g+7 (read by the next group's panels) and list 4 ("rest")
   // the others, with all four steps.  9 ints per item: target slot, then per
   // step the staged A and B indices or -1.  List l of group g:
-  // [qs_off[5g + l], qs_off[5g + l + 1]).
-  std::vector<int64_t> qs_off;
+  // [qs_off[5g + l], qs_off[5g + l + 1]), with qs_products[5g + l] products.
+  // The items are on the host until the upload.
+  std::vector<int64_t> qs_off, qs_products;
   std::vector<int32_t> qs_items;
   // Device copies.
   int32_t *d_perm = nullptr, *d_pinv = nullptr, *d_slot = nullptr;
@@ -73,4 +74,5 @@ void plan_free_device(aosb_plan* p);
 void solve_graphs_forget(const aosb_plan* p);
 void build_super_steps(aosb_plan* p);
 void build_quad_steps(aosb_plan* p);
+bool four_steps_for(const aosb_plan* p, int64_t n_pencils);
 }  // namespace aosb

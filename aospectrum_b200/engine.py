@@ -487,14 +487,16 @@ class BandEngine:
                     y.data_ptr(), y.stride(0), self._stream())
         return y
 
-    def pencil_bytes(self, n_rhs: int) -> int:
+    def pencil_bytes(self, n_rhs: int, pencils: int = 1) -> int:
+        """Device bytes of a batch of ``pencils``."""
         info = self.plan.info
         lib = native.library()
         per = lib.aosb_factor_bytes(self.plan.handle, 1) + 4 * info.n_pad + 4
         per += 8 * info.n_pad * n_rhs * 2          # normal + adjoint solve blocks (complex64)
         per += 16 * self.n * n_rhs * 3             # x, r and adjoint x (complex128)
-        per += lib.aosb_factor_workspace_bytes(self.plan.handle, 1, native.PRECISION_BF16X3)
-        return int(per)
+        staging = lib.aosb_factor_workspace_bytes(self.plan.handle, pencils,
+                                                  native.PRECISION_BF16X3)
+        return int(per) * pencils + int(staging)
 
     def max_pencils(self, n_rhs: int, wanted: int | None = None) -> int:
         """Pencils that a batch may hold, at most ``wanted`` if given."""
@@ -502,14 +504,25 @@ class BandEngine:
         if self.engine.max_pencils:
             return min(self.engine.max_pencils, wanted or self.engine.max_pencils)
         wanted = min(wanted or 4096, 4096)
-        each = max(1, self.pencil_bytes(n_rhs))
+        needed = self.pencil_bytes(n_rhs, wanted)
         # blocks the caching allocator holds but nobody uses are free for us;
         # where they already suffice the device is not asked for its free
         # memory (2.7 ms, a third of a call on a small bundle)
         free = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
-        if int(free * self.engine.memory_fraction) // each < wanted:
+        if int(free * self.engine.memory_fraction) < needed:
             free += torch.cuda.mem_get_info(self.device)[0]
-        return max(1, min(wanted, int(free * self.engine.memory_fraction) // each))
+        budget = int(free * self.engine.memory_fraction)
+        if needed <= budget:
+            return wanted
+        # larger batches may take more staging a pencil: bisect
+        low, high = 1, wanted
+        while high - low > 1:
+            mid = (low + high) // 2
+            if self.pencil_bytes(n_rhs, mid) <= budget:
+                low = mid
+            else:
+                high = mid
+        return low
 
     # ------------------------------------------------------------- public API
     def load_values(self, h_values, s_values) -> None:

@@ -442,12 +442,12 @@ def _gpu_footprint(req: BandRequest, res: Any, kpoints_per_unit: int) -> tuple[i
     L, M = st.block_size, st.moment_size
     per_pencil = (lib.aosb_factor_bytes(res.plan.handle, 1) + 4 * info.n_pad + 4
                   + 8 * info.n_pad * L * 2 + 16 * info.n * L * 3
-                  + lib.aosb_factor_workspace_bytes(res.plan.handle, 1, native.PRECISION_BF16X3)
                   + lib.aosb_solve_scratch_bytes(res.plan.handle, 1, L))
     nk = kpoints_per_unit
     pencils = nk * _pairs_per_k(st)
     per_k = 2 * 8 * info.nnz + 16 * info.n * (L * M * 2 + L)   # H, S values, moments, rhs
     working = pencils * per_pencil + nk * per_k + 64 * 2**20   # + small buffers and slack
+    working += lib.aosb_factor_workspace_bytes(res.plan.handle, pencils, native.PRECISION_BF16X3)
     return res.resident_bytes(), int(working)
 
 

@@ -312,8 +312,9 @@ typedef struct {
 
 size_t aosb_factor_bytes(const aosb_plan_t *plan, int32_t n_pencils);
 /* Tensor-core precisions: four staging buffers of split-BF16 panel tiles
- * (eight for plans of at least 500 tile products a step, which take four steps
- * at a time) plus 256 bytes for the item counter that an update's main and
+ * (eight for batches that take four steps at a time: plans of at least 500 tile
+ * products a step, batches of at least 10,000 over all pencils; a pencil's
+ * rounding so depends on how many are factored with it) plus 256 bytes for the item counter that an update's main and
  * lookahead launches share; 0 for precision 0.  A workspace sized for
  * n_pencils serves any batch of at most n_pencils; one factorization at a
  * time per workspace. */
