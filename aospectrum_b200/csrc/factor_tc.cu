@@ -788,8 +788,17 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
   // chain is done, so a generous reserve costs little.  1000-atom cube, ms a
   // factorization with 5/4 SM a pencil / a third: 1 pencil 23.4 / 17.3, 4: 51.4
   // / 36.3, 8: 81.9 / 67.9, 16: 130.7 / 131.2, 32 and 64 alike; 343 atoms, 13
-  // orbitals, 4 pencils: 9.7 / 6.7.
-  const int reserve = !lookahead ? 0 : chosen > 0 ? std::min(chosen, sms / 2) : sms / 3;
+  // orbitals, 4 pencils: 9.7 / 6.7.  In the one-step form the reserved SMs do not
+  // join, so from 8,000 tile products a step over all pencils on, where the rest
+  // update outlasts the chain, it keeps 5/4 SM a pencil.  There, 1000-atom cube, 4
+  // pencils 51.7 / 45.1, 8: 87.3 / 87.4, 16: 159 / 172, 32: 336 / 347; 343 atoms,
+  // 16 pencils 16.0 / 15.1, 32: 28.3 / 28.9.
+  const bool long_rest = a->precision == AOSB_PRECISION_BF16X3_ONE_STEP &&
+                         P->schur_updates * np >= 8000 * P->nb;
+  const int reserve = !lookahead  ? 0
+                      : chosen > 0 ? std::min(chosen, sms / 2)
+                      : long_rest  ? std::min(std::max(np * 5 / 4, 8), sms / 3)
+                                   : sms / 3;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_cross = nullptr, ev_panel = nullptr;
   if (lookahead) {

@@ -325,7 +325,9 @@ int aosb_factor(const aosb_plan_t *plan, const aosb_factor_args_v1 *args,
 /* SMs that the tensor-core factorization leaves to its lookahead side
  * stream (next steps' diagonal LU, panel products and staging) while the
  * Schur update runs on the others; 0 restores the default, a third of the
- * SMs; values are capped at SMs / 2.
+ * SMs (precision 3 with at least 8,000 tile products a step over all pencils:
+ * 5/4 of the pencils, at least 8, at most a third); values are capped at
+ * SMs / 2.
  * Process-wide; returns the previous setting (-1 for sms < 0).  No
  * counterpart in the reference (cuDSS schedules internally). */
 int32_t aosb_factor_set_lookahead_sms(int32_t sms);
