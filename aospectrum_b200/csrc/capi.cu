@@ -11,6 +11,7 @@
 //     complex64 refinement steps, aospectrum_cudss_complex64_ubatch.c:375).
 #include "plan.h"
 #include "factor.h"
+#include "side_stream.h"
 
 #include <atomic>
 #include <chrono>

@@ -14,6 +14,7 @@
 #include "cgemm.cuh"
 #include "diag_lu.cuh"
 #include "factor.h"
+#include "side_stream.h"
 
 namespace aosb {
 namespace {
@@ -409,14 +410,8 @@ template <int T>
 int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap, bool real,
               float* diag_tiles) {
   if (int rc = ensure_diag_attr<T>(err, cap)) return rc;
-  cudaStream_t st = (cudaStream_t)a->stream, side = nullptr;
-  struct Events {
-    cudaEvent_t ready = nullptr, done = nullptr;
-    ~Events() {
-      if (ready) cudaEventDestroy(ready);
-      if (done) cudaEventDestroy(done);
-    }
-  } ev;
+  cudaStream_t st = (cudaStream_t)a->stream;
+  SideWork work;
   step_diag<T>(P, a, 0, st, real, diag_tiles);
   for (int64_t k = 0; k < P->nb; ++k) {
     step_panels<T>(P, a, k, real);
@@ -429,21 +424,16 @@ int run_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
       if (next) step_diag<T>(P, a, k + 1, st, real, diag_tiles);
       continue;
     }
-    if (side == nullptr) {
-      if (int rc = side_stream(st, &side, err, cap)) return rc;
-      AOSB_CUDA_TRY(cudaEventCreateWithFlags(&ev.ready, cudaEventDisableTiming), err, cap);
-      AOSB_CUDA_TRY(cudaEventCreateWithFlags(&ev.done, cudaEventDisableTiming), err, cap);
-    }
+    if (work.stream == nullptr)
+      if (int rc = work.open(st, kSideFactor, err, cap)) return rc;
     // the lists are in tile order, so tile (k + 1, k + 1) is the first target
     const bool leads = P->lb_tile[P->lb_off[k]] == k + 1 && P->ur_tile[P->ur_off[k]] == k + 1;
     const int64_t head = leads ? 1 : 0;
     if (int rc = launch_schur<T>(P, a, k, nU, 0, head, real, err, cap)) return rc;
-    AOSB_CUDA_TRY(cudaEventRecord(ev.ready, st), err, cap);
-    AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev.ready, 0), err, cap);
-    step_diag<T>(P, a, k + 1, side, real, diag_tiles);
-    AOSB_CUDA_TRY(cudaEventRecord(ev.done, side), err, cap);
+    if (int rc = work.fork(err, cap)) return rc;
+    step_diag<T>(P, a, k + 1, work.stream, real, diag_tiles);
     if (int rc = launch_schur<T>(P, a, k, nU, head, targets - head, real, err, cap)) return rc;
-    AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev.done, 0), err, cap);
+    if (int rc = work.join(err, cap)) return rc;
   }
   return launch_check(err, cap, "plain factorization");
 }

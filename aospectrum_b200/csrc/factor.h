@@ -17,11 +17,6 @@ int factor_step_diag(const aosb_plan* P, const aosb_factor_args_v1* a, int k, cu
 // complement that the steps before left.
 int factor_plain(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap,
                  bool real = false, float* diag_tiles = nullptr);
-// Side stream of a caller stream for the lookahead (created once, non-blocking,
-// of the highest priority, kept for the life of the process or until the owner of
-// the caller stream gives it back, which it does before it destroys its stream).
-int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap);
-void side_stream_forget(cudaStream_t main);
 int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_t cap);
 size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils);
 // Two-CTA (M = 256) Schur update of one pair list (schur_pair.cu): the

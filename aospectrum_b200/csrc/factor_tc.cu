@@ -31,6 +31,7 @@
 //   still frees its TMEM.
 #include "plan.h"
 #include "factor.h"
+#include "side_stream.h"
 #include "cgemm.cuh"
 #include "tc_common.cuh"
 #include "timing.h"
@@ -40,7 +41,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <mutex>
 #include <vector>
 
 namespace aosb {
@@ -684,42 +684,6 @@ size_t factor_tc_workspace(const aosb_plan* P, int32_t n_pencils) {
          kClaimBytes;
 }
 
-namespace {
-std::mutex g_side_mutex;
-std::vector<std::pair<cudaStream_t, cudaStream_t>> g_side_streams;  // (caller's, side)
-}  // namespace
-
-int side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap) {
-  int device = 0;
-  cudaGetDevice(&device);
-  std::lock_guard<std::mutex> lock(g_side_mutex);
-  for (auto& e : g_side_streams) {
-    if (e.first == main) {
-      int dev2 = -1;
-      if (cudaStreamGetDevice(e.second, &dev2) == cudaSuccess && dev2 == device) {
-        *out = e.second;
-        return 0;
-      }
-    }
-  }
-  cudaStream_t s = nullptr;
-  int least = 0, greatest = 0;
-  AOSB_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest), err, cap);
-  AOSB_CUDA_TRY(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest), err, cap);
-  g_side_streams.emplace_back(main, s);
-  *out = s;
-  return 0;
-}
-
-void side_stream_forget(cudaStream_t main) {
-  std::lock_guard<std::mutex> lock(g_side_mutex);
-  for (size_t i = g_side_streams.size(); i-- > 0;) {
-    if (g_side_streams[i].first != main) continue;
-    cudaStreamDestroy(g_side_streams[i].second);
-    g_side_streams.erase(g_side_streams.begin() + (std::ptrdiff_t)i);
-  }
-}
-
 // Tensor map of the factor storage as a [rows][T] FP32 matrix (each tile is
 // 2 planes x T rows), 32 x 32 boxes, 128-byte swizzle: the destination of
 // the epilogue's bulk reduce-add and store.
@@ -799,23 +763,10 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
                       : chosen > 0 ? std::min(chosen, sms / 2)
                       : long_rest  ? std::min(std::max(np * 5 / 4, 8), sms / 3)
                                    : sms / 3;
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_cross = nullptr, ev_panel = nullptr;
-  if (lookahead) {
-    if (int rc = side_stream(st, &side, err, cap)) return rc;
-    AOSB_CUDA_TRY(cudaEventCreateWithFlags(&ev_cross, cudaEventDisableTiming), err, cap);
-    if (cudaEventCreateWithFlags(&ev_panel, cudaEventDisableTiming) != cudaSuccess) {
-      cudaEventDestroy(ev_cross);
-      return set_error(err, cap, AOSB_ERR_CUDA, "cudaEventCreate failed");
-    }
-  }
-  struct EventGuard {
-    cudaEvent_t a, b;
-    ~EventGuard() {
-      if (a) cudaEventDestroy(a);
-      if (b) cudaEventDestroy(b);
-    }
-  } guard{ev_cross, ev_panel};
+  SideWork work;
+  if (lookahead)
+    if (int rc = work.open(st, kSideFactor, err, cap)) return rc;
+  const cudaStream_t side = work.stream;
   const int64_t buffer_bytes = (int64_t)np * pencil_stride;
   const int n_buffers = stage_buffers(P, np);
   auto stage_buf = [&](int64_t k) { return staging + (k % n_buffers) * buffer_bytes; };
@@ -1006,13 +957,11 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     for (int64_t g = 0; kMaxSteps * (g + 1) < nb; ++g) {
       four_step(g, kMaxSteps - 1, sms, st);
       AOSB_CUDA_TRY(cudaMemsetAsync(claim_counter, 0, sizeof(int), st), err, cap);
-      AOSB_CUDA_TRY(cudaEventRecord(ev_cross, st), err, cap);
-      AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_cross, 0), err, cap);
+      if (int rc = work.fork(err, cap)) return rc;
       if (int rc = prepare(g + 1, side, reserve)) return rc;
       four_step(g, kMaxSteps, sms - reserve, st, claim_counter, true);
       four_step(g, kMaxSteps, reserve, side, claim_counter, false);
-      AOSB_CUDA_TRY(cudaEventRecord(ev_panel, side), err, cap);
-      AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev_panel, 0), err, cap);
+      if (int rc = work.join(err, cap)) return rc;
     }
     return launch_check(err, cap, "tensor-core factorization");
   }
@@ -1031,8 +980,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
         // sms - reserve SMs starts at once, a second launch on the reserved
         // SMs joins it once the side stream's panel work is done
         AOSB_CUDA_TRY(cudaMemsetAsync(claim_counter, 0, sizeof(int), st), err, cap);
-        AOSB_CUDA_TRY(cudaEventRecord(ev_cross, st), err, cap);
-        AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_cross, 0), err, cap);
+        if (int rc = work.fork(err, cap)) return rc;
         if (int rc = panels(k2, side, reserve)) return rc;
         if (k3 < nb) {
           inner(k2, side, reserve);
@@ -1043,8 +991,7 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
         // items
         two_step(ss, false, sms - reserve, st, claim_counter, true);
         two_step(ss, false, reserve, side, claim_counter, false);
-        AOSB_CUDA_TRY(cudaEventRecord(ev_panel, side), err, cap);
-        AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev_panel, 0), err, cap);
+        if (int rc = work.join(err, cap)) return rc;
       } else {
         two_step(ss, false, sms);
       }
@@ -1087,12 +1034,10 @@ int factor_tc(const aosb_plan* P, const aosb_factor_args_v1* a, char* err, size_
     const int rest = (nL - a0) * (nU - b0);
     const int cross = nL * nU - rest;
     if (cross > 0) schur(k, kMapCross, a0, b0, cross, sms);
-    AOSB_CUDA_TRY(cudaEventRecord(ev_cross, st), err, cap);
-    AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_cross, 0), err, cap);
+    if (int rc = work.fork(err, cap)) return rc;
     if (int rc = panels(k + 1, side, reserve)) return rc;
-    AOSB_CUDA_TRY(cudaEventRecord(ev_panel, side), err, cap);
     if (rest > 0) schur(k, kMapRest, a0, b0, rest, sms - reserve);
-    AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev_panel, 0), err, cap);
+    if (int rc = work.join(err, cap)) return rc;
   }
   return launch_check(err, cap, "tensor-core factorization");
 }

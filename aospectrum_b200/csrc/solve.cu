@@ -13,6 +13,7 @@
 // Each sweep is right-looking: a diagonal kernel per step, then an update
 // kernel for every off-diagonal tile of that step.
 #include "plan.h"
+#include "side_stream.h"
 #include "solve_cluster.h"
 #include "cgemm.cuh"
 #include "dmma.cuh"
@@ -71,30 +72,6 @@ static ScratchLayout scratch_layout(const aosb_plan* P, int np, int nrhs, void* 
   }
   l.bytes = off;
   return l;
-}
-
-// Side stream of a caller stream for the solve lookahead (created once,
-// non-blocking, kept for the life of the process).
-static int solve_side_stream(cudaStream_t main, cudaStream_t* out, char* err, size_t cap) {
-  static std::mutex mu;
-  static std::vector<std::pair<cudaStream_t, cudaStream_t>> table;
-  int device = 0;
-  cudaGetDevice(&device);
-  std::lock_guard<std::mutex> lock(mu);
-  for (auto& e : table) {
-    if (e.first == main) {
-      int dev2 = -1;
-      if (cudaStreamGetDevice(e.second, &dev2) == cudaSuccess && dev2 == device) {
-        *out = e.second;
-        return 0;
-      }
-    }
-  }
-  cudaStream_t s = nullptr;
-  AOSB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), err, cap);
-  table.emplace_back(main, s);
-  *out = s;
-  return 0;
 }
 
 namespace {
@@ -688,23 +665,9 @@ int run_solve(const aosb_plan* P, const aosb_solve_args_v1* a, char* err, size_t
   };
   const int nb = (int)P->nb;
   const bool lookahead = tc && g_solve_lookahead.load() != 0 && nb > 1;
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_next = nullptr, ev_diag = nullptr;
-  if (lookahead) {
-    if (int rc = solve_side_stream(st, &side, err, cap)) return rc;
-    AOSB_CUDA_TRY(cudaEventCreateWithFlags(&ev_next, cudaEventDisableTiming), err, cap);
-    if (cudaEventCreateWithFlags(&ev_diag, cudaEventDisableTiming) != cudaSuccess) {
-      cudaEventDestroy(ev_next);
-      return set_error(err, cap, AOSB_ERR_CUDA, "cudaEventCreate failed");
-    }
-  }
-  struct EventGuard {
-    cudaEvent_t a, b;
-    ~EventGuard() {
-      if (a) cudaEventDestroy(a);
-      if (b) cudaEventDestroy(b);
-    }
-  } guard{ev_next, ev_diag};
+  SideWork work;
+  if (lookahead)
+    if (int rc = work.open(st, kSideSolve, err, cap)) return rc;
   // One sweep over the steps in `order`: without lookahead, per step the
   // diagonal solve and then all updates.  With lookahead, step k first
   // updates the tile of the next step (the first list entry going forward,
@@ -733,12 +696,10 @@ int run_solve(const aosb_plan* P, const aosb_solve_args_v1* a, char* err, size_t
         if (forward && e > b && host_tiles[b] == kn) { nb1 = b + 1; rb = b + 1; }
         if (!forward && e > b && host_tiles[e - 1] == kn) { nb0 = e - 1; nb1 = e; re = e - 1; }
         update(k, nb0, nb1, dtiles, dslots, uop, buf, false);
-        AOSB_CUDA_TRY(cudaEventRecord(ev_next, st), err, cap);
-        AOSB_CUDA_TRY(cudaStreamWaitEvent(side, ev_next, 0), err, cap);
-        diag(kn, dop, buf ^ 1, side);
-        AOSB_CUDA_TRY(cudaEventRecord(ev_diag, side), err, cap);
+        if (int rc = work.fork(err, cap)) return rc;
+        diag(kn, dop, buf ^ 1, work.stream);
         update(k, rb, re, dtiles, dslots, uop, buf, true);
-        AOSB_CUDA_TRY(cudaStreamWaitEvent(st, ev_diag, 0), err, cap);
+        if (int rc = work.join(err, cap)) return rc;
       } else {
         update(k, b, e, dtiles, dslots, uop, buf, true);
       }

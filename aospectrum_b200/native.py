@@ -144,6 +144,7 @@ _SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
     "aosb_factor_workspace_bytes": (c_sz, [c_vp, c_i32, c_i32]),
     "aosb_factor_set_lookahead_sms": (c_i32, [c_i32]),
     "aosb_tc_set_wait_limit": (c_i64, [c_i64]),
+    "aosb_stream_release": (c_i32, [c_vp]),
     "aosb_factor_set_schur_pairs": (c_i32, [c_i32]),
     "aosb_solve_set_ctas_per_sm": (c_i32, [c_i32]),
     "aosb_solve_set_lookahead": (c_i32, [c_i32]),

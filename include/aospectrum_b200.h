@@ -322,6 +322,12 @@ size_t aosb_factor_workspace_bytes(const aosb_plan_t *plan, int32_t n_pencils,
                                    int32_t precision);
 int aosb_factor(const aosb_plan_t *plan, const aosb_factor_args_v1 *args,
                 char *err, size_t err_cap);
+/* aosb_factor and the solve lookahead run part of their work on a side stream
+ * that is kept with the caller's stream.  Call this before destroying a stream
+ * that was given to them, when no other thread is using it: the side streams
+ * are given back (work on them still completes, and the stream can be used
+ * again, which makes new ones).  Returns how many there were. */
+int32_t aosb_stream_release(void *stream);
 /* SMs that the tensor-core factorization leaves to its lookahead side
  * stream (next steps' diagonal LU, panel products and staging) while the
  * Schur update runs on the others; 0 restores the default, a third of the
