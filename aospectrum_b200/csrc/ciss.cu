@@ -9,6 +9,7 @@
 #include "dmma.cuh"
 #include "timing.h"
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -173,15 +174,17 @@ __global__ void gram_reduce_kernel(int chunks, int64_t pq, const double2* __rest
 // y (n x r) = x (n x p) t (p x r): a warp owns 16 rows x 32 columns, a CTA 64
 // rows, on FP64 matrix instructions with fragments straight from global memory
 // (t stays in L1 and L2).  n = 13000, p = 128, r = 104: 100 us with the former
-// shared-memory form, now 59 (floor 37 at 37 TFLOP/s).
-__global__ void __launch_bounds__(128) dense_mul_kernel(int64_t n, int p, int r,
+// shared-memory form, now 59 (floor 37 at 37 TFLOP/s).  A launch takes the
+// columns from `first` on, as many as the grid's y extent covers.
+constexpr int kDenseColumns = 32;
+__global__ void __launch_bounds__(128) dense_mul_kernel(int64_t n, int p, int r, int first,
                                                         const double2* __restrict__ x,
                                                         int64_t ldx,
                                                         const double2* __restrict__ t,
                                                         double2* __restrict__ y, int64_t ldy) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t r0 = (int64_t)blockIdx.x * 64 + warp * 16;
-  const int c0 = blockIdx.y * 32;
+  const int c0 = first + blockIdx.y * kDenseColumns;
   if (r0 >= n) return;
   const int hi = lane / 4, lo = lane % 4;
   const double2 zero = make_double2(0.0, 0.0);
@@ -376,10 +379,14 @@ int aosb_dense_mul(int64_t n, int32_t p, int32_t r, const aosb_complex128* x, in
     return aosb::set_error(err, cap, AOSB_ERR_NULL, "null argument");
   if (n <= 0 || p <= 0 || r <= 0 || ldx < p || ldy < r)
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "invalid dense_mul shape");
-  dim3 grid(aosb::ceil_div(n, 64), aosb::ceil_div(r, 32));
-  aosb::dense_mul_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(
-      n, p, r, (const double2*)x, ldx, (const double2*)t, (double2*)y, ldy);
-  aosb::count_launches(1);
+  constexpr int kMost = 65535 * aosb::kDenseColumns;  // columns of a launch: the grid's y limit
+  for (int64_t first = 0; first < r; first += kMost) {
+    dim3 grid(aosb::ceil_div(n, 64),
+              aosb::ceil_div(std::min<int64_t>(r - first, kMost), aosb::kDenseColumns));
+    aosb::dense_mul_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(
+        n, p, r, (int)first, (const double2*)x, ldx, (const double2*)t, (double2*)y, ldy);
+    aosb::count_launches(1);
+  }
   return aosb::launch_check(err, cap, "dense_mul");
 }
 
