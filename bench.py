@@ -746,6 +746,8 @@ def main() -> None:
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (
         ROOT / "MEASURED_PEAKS.json").exists() else {}
     tc = args.precision == "mixed" and bool(args.tensor_cores)
+    steps_at_a_time = schur_steps(info, float(np.mean(eng.factor_pencils or [1])),
+                                  eng.engine.schur_depth, bool(pairs_on))
     ft = eng.factor_times_ms
     factor_tflops = (info.factor_flops_alg * float(np.mean(eng.factor_pencils)) /
                      (float(np.mean(ft)) / 1e3) / 1e12) if ft else None
@@ -757,9 +759,7 @@ def main() -> None:
         peak = sustained if sustained else 1400.0
         achieved = k_flops.value / (k_ms.value / 1e3) / 1e12
         per_launch_units = k_flops.value / k_launches.value / (8.0 * info.tile ** 3)
-        # c2 takes four steps at a time from 8 pencils on
-        traffic = schur_traffic_per_unit(
-            "four" if np.mean(eng.factor_pencils or [1]) >= 8 and not args.schur_pairs else "two")
+        traffic = schur_traffic_per_unit(steps_at_a_time)
         roofline = {
             "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak,
@@ -801,7 +801,7 @@ def main() -> None:
                    else 0,
                    "tensor_core_solves": bool(eng.engine.tensor_core_solves),
                    "cuda_graphs": bool(eng.engine.cuda_graphs),
-                   "schur_depth": eng.engine.schur_depth,
+                   "schur_depth": steps_at_a_time,
                    "schur_pairs": bool(pairs_on),
                    "solve_lookahead": bool(look_on),
                    "lookahead_sms": args.lookahead_sms or "default",
@@ -936,12 +936,24 @@ def main() -> None:
         dist.destroy_process_group()
 
 
-def schur_traffic_per_unit(steps: str) -> dict | None:
+def schur_steps(info, pencils: float, depth: int, pairs: bool) -> int:
+    """Tile steps that a Schur update of a batch applies at a time: four on
+    plans of at least 500 tile products a step in batches of at least 10,000
+    (not in the two-CTA form), else as many as the engine's depth."""
+    products = info.schur_tile_updates / info.n_tiles
+    if depth == 2 and not pairs and products >= 500 and products * pencils >= 10000:
+        return 4
+    return depth
+
+
+def schur_traffic_per_unit(steps: int) -> dict | None:
     """DRAM bytes per algorithmic unit of schur_tc_kernel -- one (target
     tile, tile step, pencil) update, 8 T^3 flops -- from the committed ncu
     capture summary of the two- or four-step kernel (dram__bytes_read.sum +
-    write.sum of the captured launch divided by the units it applied)."""
-    f = ROOT / "profiles" / f"schur_tc_kernel_{steps}_step_c2.json"
+    write.sum of the captured launch divided by the units it applied); None
+    for a form without a capture."""
+    name = {2: "two", 4: "four"}.get(steps, steps)
+    f = ROOT / "profiles" / f"schur_tc_kernel_{name}_step_c2.json"
     if not f.exists():
         return None
     d = json.loads(f.read_text())
