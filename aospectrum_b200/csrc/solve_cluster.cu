@@ -544,9 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       } else {
         consumers_any(false);  // order[] is written
       }
-      // Each lane polls for itself, so a wait may run out in some lanes of a warp
-      // only; the warp goes on by one verdict, since the unit loop below votes.
-      ok = __all_sync(0xffffffffu, cluster_wait(&sh.bar_y, phase, a.limit) ? 1 : 0);
+      ok = cluster_wait(&sh.bar_y, phase, a.limit);
 #pragma unroll
       for (int o = 0; o < kPairs; ++o) {
         const int i = 2 * (warp + kWarps * o);
@@ -560,7 +558,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       // update units of this CTA, in turn to the groups of warps
       for (int u = rank, j = 0; u < units; u += C, ++g, ++j) {
         if (j % kGroups != group) continue;
-        if (ok) ok = __all_sync(0xffffffffu, entry_ready(g) ? 1 : 0);
+        // Each lane polls for itself, so a wait may run out in some lanes of a
+        // warp only: all of them vote, those that gave up above among them.
+        ok = __all_sync(0xffffffffu, ok && entry_ready(g) ? 1 : 0);
         // after a failure both warps of a pair still meet
         if (!ok) {
           pair_sync(2 + group * 2 + (warp & 1));
