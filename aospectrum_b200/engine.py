@@ -103,6 +103,7 @@ class PlanSummary:
     factor_flops: float
     factor_flops_alg: float
     factor_bytes: float
+    schur_tile_updates: int
 
 
 class BlochDevice:
@@ -235,7 +236,8 @@ class SymbolicPlan:
         self.ordering = "nested_dissection" if mode == 1 else "natural"
         self.info = PlanSummary(info.n, info.n_pad, info.nnz, info.tile, info.n_tiles,
                                 info.n_slots, info.n_nodes, info.tree_levels, info.factor_flops,
-                                info.factor_flops_alg, info.factor_bytes)
+                                info.factor_flops_alg, info.factor_bytes,
+                                info.schur_tile_updates)
         self.device = device
         if upload:
             self.upload()
