@@ -98,7 +98,8 @@ class EngineSettings:
         refinement recovers the accuracy); False keeps them in FP32 SIMT.
     schur_depth: 2 applies the Schur updates of two tile steps in one
         tensor-core pass (K = 256: each target tile read and written once per
-        two steps); 1 updates after every step.
+        two steps), and of four where plan and batch are large enough for that
+        to pay; 1 updates after every step.
     cuda_graphs: capture each batch's triangular sweeps (hundreds of
         launches per solve) into a CUDA graph on first use and replay it.
     autotune: with tile 0, time the candidate tile plans (tile edge x

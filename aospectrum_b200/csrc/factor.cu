@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(kThreads) schur_words_kernel(
 // Schur update of 64- and 128-wide tiles: blockIdx.x = (pair, 64 x 64 part),
 // blockIdx.y = pencil.  128 threads own 8 x 4 complex elements each (rows 8
 // apart), so a K step of four reads 24 16-byte words of shared memory for 512
-// FMAs and the FP32 pipe is the bound; the operands come as they lie in the
-// tiles by cp.async, two K slices of 16 deep, and four CTAs fit an SM.  The
-// former 4 x 4 form with scalar words and slices staged through registers ran
+// FMAs and issue is the bound (2304 CTAs: 2.9 instructions a cycle, FMA pipe
+// 66 %); the operands come as they lie in the tiles by cp.async, two K slices of
+// 16 deep, and four CTAs fit an SM.  The former 4 x 4 form with scalar words and slices staged through registers ran
 // at a third of the FP32 rate: 8 pencils of the 343-atom cube (5 orbitals) 88
 // us a step, now 72; 70 tiles of 64, one pencil: 71 us, now 59.
 // Real pencils (the imaginary planes are zero and stay so) take a quarter of

@@ -709,7 +709,7 @@ Residency residency(int device) {
 // Microseconds of one step of `units` units in a form: the chain of a step,
 // the diagonal product over its CTAs, the update units of the busiest CTA, all
 // times the waves of clusters.  Fitted to whole solves of plans of 7 to 114
-// tiles with 16 to 600 units; us a step, 32 columns, this kernel / one launch
+// steps with 16 to 600 units; us a step, 32 columns, this kernel / one launch
 // per step: 1000-atom bundle (102 steps) 8 pencils 30 / 41, 16: 47 / 56, 32: 63
 // / 84, 64: 119 / 142; 64 atoms (7 steps), 5 pencils 10 / 32, 16: 16 / 42, 300:
 // 133 / 347.  The waves are what loses: past one wave of the smallest clusters
@@ -728,7 +728,7 @@ double step_cost(const Form& f, int resident, int units, double tiles, int colum
 // The same for one launch per diagonal step and one per update, where the
 // columns hardly matter (102 steps, 96 pencils: 200 us with 32, 191 with 8).
 // With these two costs the form taken was at most 2 % behind the better one in
-// a hundred measured batches; with 0.85 + 0.027 tiles, and a factor of 1 for the
+// 140 batches on nine plans of up to 416 steps; with 0.85 + 0.027 tiles, and a factor of 1 for the
 // clusters, it was up to 7 % behind (108 pencils above).
 double launch_cost(int units, double tiles) { return 27.0 + units * (0.35 + 0.042 * tiles); }
 
