@@ -8,11 +8,11 @@
 // CSR arrays, because every row of atom i has the same column structure.
 // Entry (a, c) of group (i, j) sits at dst_base + a * rowlen_i + c.
 //
-// The device kernel gives a CTA a strip of up to eight neighbouring windows of
-// one row atom and all k points (in chunks of four): it sums the member blocks
-// of (i, j) and of its mirror (j, i) in block order (the order the reference's
-// stable sort leaves them in), applies the Hermitian projection of
-// sparse.py:25-36 and writes the strip row by row.  With
+// Two device kernels sum the member blocks of (i, j) and of its mirror (j, i) in
+// block order (the order the reference's stable sort leaves them in) and apply
+// the Hermitian projection of sparse.py:25-36: one gives a CTA a strip of up to
+// eight neighbouring windows of one row atom and writes it row by row, the other
+// gives a warp a window (which one when: strips_pay).  With
 // real block values the products v * phase are exact, so the output is
 // bit-identical to the reference's numpy path.
 #include "common.cuh"
@@ -21,6 +21,12 @@
 #include <algorithm>
 #include <numeric>
 #include <vector>
+
+// The windows in strips, the mean windows, columns and values of a strip, and the
+// mean of its largest window's values over its mean window's.
+struct StripShape {
+  double windows = 0, per_strip = 0, columns = 0, values = 0, uneven = 0;
+};
 
 struct aosb_bloch {
   int64_t n = 0, n_atoms = 0, n_blocks = 0, nnz = 0;
@@ -38,6 +44,7 @@ struct aosb_bloch {
   int64_t* d_member_off = nullptr; // value offset of each member block
   int32_t* d_member_shift = nullptr;
   int2* d_strips = nullptr;        // [first, last) groups of each strip
+  int32_t* d_others = nullptr;     // groups in no strip
   // host copies of the device tables (uploaded by aosb_bloch_upload)
   std::vector<int4> g_info;
   std::vector<int64_t> g_dst;
@@ -45,6 +52,8 @@ struct aosb_bloch {
   std::vector<int64_t> m_off;
   std::vector<int32_t> m_shift;
   std::vector<int2> strips;
+  std::vector<int32_t> others;
+  StripShape shape;
   int64_t n_values = 0;  // stored block values (sum of block sizes), set at upload
   bool uploaded = false;
 };
@@ -123,7 +132,8 @@ __device__ __forceinline__ float2 hermitian_mean(float2 x, float2 y) {
 
 // Strips: neighbouring windows (i, j) of one row atom, whose segments of each
 // CSR row are contiguous; at most kStripWindows of them, kStripColumns columns
-// and kStripValues elements (a longer window is a strip of its own).
+// and kStripValues elements, and one member block each way in every window (a
+// single lattice image).  Windows that do not fit belong to no strip.
 constexpr int kStripWindows = 8, kStripColumns = 128, kStripValues = 1376;
 constexpr int kStripThreads = 256;
 
@@ -134,62 +144,152 @@ constexpr int kStripThreads = 256;
 // elements above and below the diagonal do so, and the diagonal keeps its real
 // part.
 
-// One warp, one window, any number of member blocks.
+// One warp, one window: any number of member blocks, any size.
 template <typename V>
-__device__ __forceinline__ void window_sums(int g, int lane, int k0, int nk,
-                                            const int4* __restrict__ group,
-                                            const int64_t* __restrict__ gdst,
-                                            const int2* __restrict__ gmem,
-                                            const int64_t* __restrict__ moff,
-                                            const int32_t* __restrict__ msh,
-                                            const V* __restrict__ hv, const V* __restrict__ sv,
-                                            const float2* __restrict__ phases, int64_t n_shifts,
-                                            int64_t nnz, float2* __restrict__ hout,
-                                            float2* __restrict__ sout) {
+__device__ __forceinline__ void window_sums(
+    int g, int lane, int k0, int n_k, const int4* __restrict__ group,
+    const int64_t* __restrict__ gdst, const int2* __restrict__ gmem,
+    const int64_t* __restrict__ moff, const int32_t* __restrict__ msh, const V* __restrict__ hv,
+    const V* __restrict__ sv, const float2* __restrict__ phases, int64_t n_shifts, int64_t nnz,
+    float2* __restrict__ hout, float2* __restrict__ sout) {
+  const int nk = min(n_k - k0, kBlochKChunk);
   const float2* ph0 = phases + (int64_t)k0 * n_shifts;
+  const int64_t out0 = (int64_t)k0 * nnz;
   const int4 gi = group[g];  // nr, nc, rowlen, mirror
   const int nr = gi.x, nc = gi.y, rl = gi.z, gm = gi.w;
   const int ne = nr * nc;
-  const int64_t at0 = (int64_t)k0 * nnz + gdst[g];
-  const int2 rg = gmem[g], mr = gmem[gm];
+  const int64_t base = gdst[g];
+  const int2 rg = gmem[g];
   float2 x[kBlochKChunk], y[kBlochKChunk];
-  // t runs over [matrix H|S][row-major element]
+  if (gm == g) {
+    // diagonal window: t runs over [matrix H|S][row-major element]; the mean
+    // of the pair (lo, hi) is formed the same way for both of its entries
+    for (int t = lane; t < 2 * ne; t += 32) {
+      const int which = t >= ne;
+      const int e = t - which * ne;
+      const int a = e / nc, c = e - (e / nc) * nc;
+      const V* vals = which == 0 ? hv : sv;
+      float2* out = (which == 0 ? hout : sout) + out0 + base + (int64_t)a * rl + c;
+      const int lo = min(a, c), hi = max(a, c);
+      group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, rg, lo * nc + hi, x);
+      if (a != c) group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, rg, hi * nc + lo, y);
+#pragma unroll
+      for (int q = 0; q < kBlochKChunk; ++q) {
+        if (q < nk) {
+          float2 v;
+          if (a == c) {
+            v = make_float2(x[q].x, 0.0f);
+          } else {
+            const float2 mean = hermitian_mean(x[q], y[q]);
+            v = a < c ? mean : make_float2(mean.x, -mean.y);
+          }
+          out[q * nnz] = v;
+        }
+      }
+    }
+    return;
+  }
+  const bool lower = gm < g;
+  const int2 mr = gmem[gm];
+  // the mean's first operand comes from the upper group of the pair
+  const int2 r1 = lower ? mr : rg, r2 = lower ? rg : mr;
+  if (r1.y - r1.x == 1 && r2.y - r2.x == 1) {
+    // One member block each way (a single lattice image, the common case):
+    // value offsets and phases are warp-uniform and loaded once; each lane
+    // keeps two elements' value loads in flight.
+    const int64_t o1 = moff[r1.x], o2 = moff[r2.x];
+    const float2* ph1 = ph0 + msh[r1.x];
+    const float2* ph2 = ph0 + msh[r2.x];
+    float2 p1[kBlochKChunk], p2[kBlochKChunk];
+#pragma unroll
+    for (int q = 0; q < kBlochKChunk; ++q) {
+      p1[q] = q < nk ? ph1[q * n_shifts] : make_float2(0.0f, 0.0f);
+      p2[q] = q < nk ? ph2[q * n_shifts] : make_float2(0.0f, 0.0f);
+    }
+    for (int t0 = lane; t0 < 2 * ne; t0 += 64) {
+      float2 v1[2], v2[2];
+      float2* out[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int t = t0 + 32 * u;
+        out[u] = nullptr;
+        v1[u] = v2[u] = make_float2(0.0f, 0.0f);
+        if (t < 2 * ne) {
+          const int which = t >= ne;
+          const int e = t - which * ne;
+          const int a = e / nc, c = e - a * nc;
+          const int eg = a * nc + c, em = c * nr + a;
+          const V* vals = which == 0 ? hv : sv;
+          out[u] = (which == 0 ? hout : sout) + out0 + base + (int64_t)a * rl + c;
+          v1[u] = load_value<V>(vals, o1 + (lower ? em : eg));
+          v2[u] = load_value<V>(vals, o2 + (lower ? eg : em));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (out[u] == nullptr) continue;
+#pragma unroll
+        for (int q = 0; q < kBlochKChunk; ++q) {
+          if (q < nk) {
+            const float2 mean = hermitian_mean(cmul_rn(v1[u], p1[q]), cmul_rn(v2[u], p2[q]));
+            out[u][q * nnz] = lower ? make_float2(mean.x, -mean.y) : mean;
+          }
+        }
+      }
+    }
+    return;
+  }
+  // general: t runs over [matrix H|S][row-major element]
   for (int t = lane; t < 2 * ne; t += 32) {
     const int which = t >= ne;
     const int e = t - which * ne;
     const int a = e / nc, c = e - a * nc;
     const int eg = a * nc + c, em = c * nr + a;
-    const bool lower = gm < g || (gm == g && a > c);
     const V* vals = which == 0 ? hv : sv;
-    float2* out = (which == 0 ? hout : sout) + at0 + (int64_t)a * rl + c;
-    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, lower ? mr : rg, lower ? em : eg, x);
-    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, lower ? rg : mr, lower ? eg : em, y);
+    float2* out = (which == 0 ? hout : sout) + out0 + base + (int64_t)a * rl + c;
+    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, r1, lower ? em : eg, x);
+    group_sums<V>(vals, moff, msh, ph0, n_shifts, nk, r2, lower ? eg : em, y);
 #pragma unroll
     for (int q = 0; q < kBlochKChunk; ++q) {
       if (q < nk) {
         const float2 mean = hermitian_mean(x[q], y[q]);
-        float2 v = lower ? make_float2(mean.x, -mean.y) : mean;
-        if (gm == g && a == c) v = make_float2(x[q].x, 0.0f);
-        out[q * nnz] = v;
+        out[q * nnz] = lower ? make_float2(mean.x, -mean.y) : mean;
       }
     }
   }
 }
 
-// One CTA per strip (x) and share of the k chunks (y).  Where every window of
-// the strip has one member block each way (a single lattice image, the common
-// case) the blocks are copied to shared memory, contiguous as they are stored,
-// with all copies in flight at once; then a thread keeps one column of the
-// strip, its window's phases in registers, and walks the rows: a warp writes
-// 256 contiguous bytes of a CSR row.  A warp per window, as before, gathered
-// single values in rounds of two per lane and was bound by their latency (43 %
-// of the copy bandwidth).  4096 atoms, 13 orbitals, 4 k points (4.6 GB): 1.60
-// ms, now 1.08 (0.70 at the copy bandwidth; streaming stores and other register
-// limits were slower); 64 atoms, 1 k point: 9.8 us, now 5.8.
+// A warp per window and chunk of k points.  Neighbouring warps write
+// neighbouring windows of the same CSR rows at the same time, so that the 32-byte
+// sectors they share are completed in L2.
+constexpr int kWindowWarps = 8;
+template <typename V>
+__global__ void __launch_bounds__(kWindowWarps * 32, 4) bloch_windows_kernel(
+    int64_t n_groups, const int4* __restrict__ group, const int64_t* __restrict__ gdst,
+    const int2* __restrict__ gmem, const int64_t* __restrict__ moff,
+    const int32_t* __restrict__ msh, const V* __restrict__ hv, const V* __restrict__ sv,
+    const float2* __restrict__ phases, int64_t n_shifts, int64_t nnz, int n_k,
+    float2* __restrict__ hout, float2* __restrict__ sout) {
+  const int64_t g = (int64_t)blockIdx.x * kWindowWarps + threadIdx.x / 32;
+  if (g < n_groups)
+    window_sums<V>((int)g, threadIdx.x % 32, blockIdx.y * kBlochKChunk, n_k, group, gdst, gmem,
+                   moff, msh, hv, sv, phases, n_shifts, nnz, hout, sout);
+}
+
+// One CTA per strip (x) and share of the k chunks (y), after `lead` CTAs with a
+// warp for each window outside strips and each chunk.  The strip's blocks are
+// copied to shared memory, contiguous as they are stored, with all copies in
+// flight at once; then a thread keeps one column of the strip, its window's
+// phases in registers, and walks the rows: a warp writes 256 contiguous bytes of
+// a CSR row, and the blocks are read once for all k.  A warp per window gathers
+// single values in rounds of two per lane and is bound by their latency (43 % of
+// the copy bandwidth).  4096 atoms, 13 orbitals, 4 k points (4.6 GB): 1.60 ms
+// with it, 1.08 here (0.70 at the copy bandwidth; streaming stores and other
+// register limits were slower); 64 atoms, 1 k point: 9.8 and 5.8 us.
 template <typename V>
 __global__ void __launch_bounds__(kStripThreads) bloch_strips_kernel(
-    const int2* __restrict__ strips, const int4* __restrict__ group,
-    const int64_t* __restrict__ gdst, const int2* __restrict__ gmem,
+    const int2* __restrict__ strips, int lead, int n_others, const int32_t* __restrict__ others,
+    const int4* __restrict__ group, const int64_t* __restrict__ gdst, const int2* __restrict__ gmem,
     const int64_t* __restrict__ moff, const int32_t* __restrict__ msh, const V* __restrict__ hv,
     const V* __restrict__ sv, const float2* __restrict__ phases, int64_t n_shifts, int64_t nnz,
     int n_k, float2* __restrict__ hout, float2* __restrict__ sout) {
@@ -197,62 +297,50 @@ __global__ void __launch_bounds__(kStripThreads) bloch_strips_kernel(
   __shared__ V vals[2][2][kStripValues];
   __shared__ int first_value[kStripWindows], first_column[kStripWindows + 1], widths[kStripWindows];
   __shared__ int mirrors[kStripWindows], own_shift[kStripWindows], mirror_shift[kStripWindows];
-  __shared__ int fast;
+  __shared__ int64_t own_offset[kStripWindows], mirror_offset[kStripWindows];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int2 st = strips[blockIdx.x];
-  const int nw = st.y - st.x;
   const int chunks = (n_k + kBlochKChunk - 1) / kBlochKChunk;
+  if ((int)blockIdx.x < lead) {
+    const int item = (int)blockIdx.x * (kStripThreads / 32) + warp;
+    if (blockIdx.y == 0 && item < n_others * chunks)
+      window_sums<V>(others[item / chunks], lane, item % chunks * kBlochKChunk, n_k, group, gdst,
+                     gmem, moff, msh, hv, sv, phases, n_shifts, nnz, hout, sout);
+    return;
+  }
+  const int2 st = strips[blockIdx.x - lead];
+  const int nw = st.y - st.x;
   if (warp == 0) {
     // window tables: one lane per window, prefix sums by shuffles
     int4 gi = make_int4(0, 0, 0, 0);
-    int2 rg = make_int2(0, 0), mr = make_int2(0, 0);
-    if (lane < nw) {
-      gi = group[st.x + lane];
-      rg = gmem[st.x + lane];
-      mr = gmem[gi.w];
-    }
+    if (lane < nw) gi = group[st.x + lane];
     int cols = gi.y, values = gi.x * gi.y;
 #pragma unroll
-    for (int o = 1; o < 32; o *= 2) {
+    for (int o = 1; o < kStripWindows; o *= 2) {
       const int c = __shfl_up_sync(0xffffffffu, cols, o), v = __shfl_up_sync(0xffffffffu, values, o);
       if (lane >= o) {
         cols += c;
         values += v;
       }
     }
-    const bool single = lane >= nw || (rg.y - rg.x == 1 && mr.y - mr.x == 1);
-    const bool all = __all_sync(0xffffffffu, single ? 1 : 0) != 0;
-    const int width = __shfl_sync(0xffffffffu, cols, 31), total = __shfl_sync(0xffffffffu, values, 31);
-    const bool ok = all && width <= kStripColumns && total <= kStripValues;
     if (lane < nw) {
       first_column[lane] = cols - gi.y;
       first_value[lane] = values - gi.x * gi.y;
       widths[lane] = gi.y;
       mirrors[lane] = gi.w;
-      if (ok) {
-        own_shift[lane] = msh[rg.x];
-        mirror_shift[lane] = msh[mr.x];
-      }
-    }
-    if (lane == 0) {
-      first_column[nw] = width;
-      fast = ok;
+      const int own = gmem[st.x + lane].x, mir = gmem[gi.w].x;
+      own_shift[lane] = msh[own];
+      mirror_shift[lane] = msh[mir];
+      own_offset[lane] = moff[own];
+      mirror_offset[lane] = moff[mir];
+      if (lane == nw - 1) first_column[nw] = cols;
     }
   }
   __syncthreads();
-  if (!fast) {
-    for (int chunk = blockIdx.y; chunk < chunks; chunk += gridDim.y)
-      for (int w = warp; w < nw; w += kStripThreads / 32)
-        window_sums<V>(st.x + w, lane, chunk * kBlochKChunk,
-                       min(n_k - chunk * kBlochKChunk, kBlochKChunk), group, gdst, gmem, moff, msh,
-                       hv, sv, phases, n_shifts, nnz, hout, sout);
-    return;
-  }
   const int4 g0 = group[st.x];
   const int nr = g0.x, rl = g0.z;
   if (warp < nw) {
     const int ne = nr * widths[warp], v0 = first_value[warp];
-    const int64_t own = moff[gmem[st.x + warp].x], mir = moff[gmem[mirrors[warp]].x];
+    const int64_t own = own_offset[warp], mir = mirror_offset[warp];
     for (int e = lane; e < ne; e += 32) {
       const V* src[4] = {hv + own + e, sv + own + e, hv + mir + e, sv + mir + e};
 #pragma unroll
@@ -305,6 +393,63 @@ __global__ void __launch_bounds__(kStripThreads) bloch_strips_kernel(
       }
     }
   }
+}
+
+// Whether the strips of a bundle take the strip kernel for n_k points (the
+// windows outside strips never do).  Strips cost a CTA with two barriers each
+// and use as many of 128 column threads as they are wide, but read their blocks
+// once and write whole rows.  They win where they are wide (13 orbitals: 8
+// windows, 104 columns); with few windows on the chip, where a warp per window
+// is bound by its own chain; where windows of one strip differ in size, which
+// leaves warps idle; and with many k points, the more so the fewer values there
+// are to load (complex blocks load twice as many).  us, a warp per window /
+// strips, 1728 atoms, real: 5 orbitals, 4 k 130 / 200, 16 k 504 / 420; 10
+// orbitals, 4 k 398 / 366; 512 atoms: 13 orbitals, 4 k 214 / 140; 20 orbitals,
+// 4 k 474 / 445, complex 492 / 502; 36 atoms (252 neighbours): 20 orbitals, 4 k 22
+// / 12; 216 atoms of 5, 14 and 25 orbitals, 4 k 154 / 95.  Over 1600 measured
+// pairs of bundle and n_k the kernel taken is 1.3 % slower than the better one
+// on average; strips for all of them were 8 %, windows 23 %.
+bool strips_pay(const StripShape& s, bool complex_values, int n_k) {
+  if (s.columns >= 88) return true;
+  const bool uneven = s.uneven >= 1.5, several = s.per_strip >= 1.5;
+  if (uneven && s.values >= 900) return true;
+  if (s.windows <= 4000) {
+    if (n_k <= 4) return s.values >= 500;
+    if (n_k <= 16) return s.values >= (s.windows <= 1500 || uneven ? 500 : 1150);
+    return n_k <= 32 && s.values >= 1150 && several;
+  }
+  if (n_k <= 4) return !complex_values && several && s.values >= (uneven ? 500 : 900);
+  if (complex_values && n_k <= 8) return several && s.values >= (uneven ? 500 : 600);
+  return s.values >= 350 || s.values <= 16 || (n_k >= 32 && !complex_values);
+}
+
+template <typename V>
+void launch_sums(const aosb_bloch* b, const void* h_values, const void* s_values,
+                 const void* phases, int n_k, void* h_out, void* s_out, cudaStream_t st) {
+  const auto *hv = (const V*)h_values, *sv = (const V*)s_values;
+  const auto* ph = (const float2*)phases;
+  auto *ho = (float2*)h_out, *so = (float2*)s_out;
+  const int64_t nsh = (int64_t)(b->shifts.size() / 3), strips = (int64_t)b->strips.size();
+  const int64_t chunks = aosb::ceil_div(n_k, kBlochKChunk), others = (int64_t)b->others.size();
+  aosb::count_launches(1);
+  // The windows outside strips run beside them while they are a few (one in
+  // fifty): a warp takes longer over one than a CTA over a strip.
+  if (others * 50 <= b->n_groups && others * chunks < INT32_MAX / 2 &&
+      strips_pay(b->shape, sizeof(V) == sizeof(float2), n_k)) {
+    // A CTA goes through all k chunks with its blocks loaded once, unless the
+    // strips alone leave SMs without eight CTAs.
+    const int64_t share = std::min<int64_t>(chunks, std::max<int64_t>(1, 148 * 8 / strips));
+    const int lead = (int)aosb::ceil_div(others * chunks, kStripThreads / 32);
+    bloch_strips_kernel<V><<<dim3((unsigned)(lead + strips), (unsigned)share), kStripThreads, 0,
+                             st>>>(b->d_strips, lead, (int)others, b->d_others, b->d_group,
+                                   b->d_group_dst, b->d_group_members, b->d_member_off,
+                                   b->d_member_shift, hv, sv, ph, nsh, b->nnz, n_k, ho, so);
+    return;
+  }
+  const dim3 grid(aosb::ceil_div(b->n_groups, kWindowWarps), (unsigned)chunks);
+  bloch_windows_kernel<V><<<grid, kWindowWarps * 32, 0, st>>>(
+      b->n_groups, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
+      b->d_member_shift, hv, sv, ph, nsh, b->nnz, n_k, ho, so);
 }
 
 }  // namespace
@@ -436,21 +581,41 @@ int aosb_bloch_create(int64_t n_orbitals, int64_t n_atoms, const int64_t* atom_o
   }
   B->n_members = (int64_t)m_off.size();
   // Strips of each row atom, of about equal window counts.
+  StripShape& shape = B->shape;
   for (int64_t a = 0; a < n_atoms; ++a) {
     const int64_t lo = first_group[a], hi = first_group[a + 1];
     const int64_t most = std::max<int64_t>(1, (hi - lo + kStripWindows - 1) / kStripWindows);
     const int64_t even = (hi - lo + most - 1) / most;
     for (int64_t g = lo; g < hi;) {
-      int64_t e = g, cols = 0, values = 0;
+      int64_t e = g, cols = 0, values = 0, largest = 0;
       while (e < hi && e - g < even) {
-        cols += g_info[e].y;
-        values += (int64_t)g_info[e].x * g_info[e].y;
-        if (e > g && (cols > kStripColumns || values > kStripValues)) break;
+        const int4 w = g_info[e];
+        const int64_t c = cols + w.y, v = values + (int64_t)w.x * w.y;
+        const bool single = g_mem[e].y - g_mem[e].x == 1 && g_mem[w.w].y - g_mem[w.w].x == 1;
+        if (!single || c > kStripColumns || v > kStripValues) break;
+        largest = std::max<int64_t>(largest, v - values);
+        cols = c;
+        values = v;
         ++e;
       }
+      if (e == g) {
+        B->others.push_back((int32_t)g++);
+        continue;
+      }
       B->strips.push_back(make_int2((int)g, (int)e));
+      shape.windows += (double)(e - g);
+      shape.columns += (double)cols;
+      shape.values += (double)values;
+      if (values > 0) shape.uneven += (double)largest * (double)(e - g) / (double)values;
       g = e;
     }
+  }
+  if (!B->strips.empty()) {
+    const double n = (double)B->strips.size();
+    shape.per_strip = shape.windows / n;
+    shape.columns /= n;
+    shape.values /= n;
+    shape.uneven /= n;
   }
   B->g_info = std::move(g_info);
   B->g_dst = std::move(g_dst);
@@ -472,7 +637,8 @@ int aosb_bloch_upload(aosb_bloch_t* B, char* err, size_t cap) {
       (rc = upload(&B->d_group_members, B->g_mem, err, cap)) ||
       (rc = upload(&B->d_member_off, B->m_off, err, cap)) ||
       (rc = upload(&B->d_member_shift, B->m_shift, err, cap)) ||
-      (rc = upload(&B->d_strips, B->strips, err, cap)))
+      (rc = upload(&B->d_strips, B->strips, err, cap)) ||
+      (rc = upload(&B->d_others, B->others, err, cap)))
     return rc;
   int64_t values = 0;
   for (size_t g = 0; g < B->g_info.size(); ++g)
@@ -543,37 +709,22 @@ int aosb_bloch_apply(const aosb_bloch_t* b, int32_t value_kind, const void* h_va
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "call aosb_bloch_upload first");
   if (n_k <= 0 || n_k > 65535)
     return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "n_k must be in 1..65535");
-  // A CTA goes through all k chunks with its blocks loaded once, unless the
-  // strips alone leave SMs without eight CTAs.
-  const int64_t strips = (int64_t)b->strips.size();
-  const int64_t chunks = aosb::ceil_div(n_k, kBlochKChunk);
-  const int64_t share = std::min<int64_t>(chunks, std::max<int64_t>(1, 148 * 8 / strips));
-  dim3 grid((unsigned)strips, (unsigned)share);
+  if (value_kind != 0 && value_kind != 1)
+    return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "value_kind must be 0 or 1");
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t nsh = (int64_t)(b->shifts.size() / 3);
   cudaEvent_t ev[2];
   const bool timed = aosb::timing_begin(st, ev);
-  if (value_kind == 0) {
-    bloch_strips_kernel<float><<<grid, kStripThreads, 0, st>>>(
-        b->d_strips, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
-        b->d_member_shift, (const float*)h_values, (const float*)s_values,
-        (const float2*)phases, nsh, b->nnz, n_k, (float2*)h_out, (float2*)s_out);
-  } else if (value_kind == 1) {
-    bloch_strips_kernel<float2><<<grid, kStripThreads, 0, st>>>(
-        b->d_strips, b->d_group, b->d_group_dst, b->d_group_members, b->d_member_off,
-        b->d_member_shift, (const float2*)h_values, (const float2*)s_values,
-        (const float2*)phases, nsh, b->nnz, n_k, (float2*)h_out, (float2*)s_out);
-  } else {
-    return aosb::set_error(err, cap, AOSB_ERR_ARGUMENT, "value_kind must be 0 or 1");
-  }
-  aosb::count_launches(1);
+  if (value_kind == 0)
+    launch_sums<float>(b, h_values, s_values, phases, n_k, h_out, s_out, st);
+  else
+    launch_sums<float2>(b, h_values, s_values, phases, n_k, h_out, s_out, st);
   // algorithmic bytes: the stored H and S block values read once per launch,
   // the complex64 H(k) and S(k) CSR values written once per k point
   if (timed)
     aosb::timing_end(aosb::kTimedBloch, st, ev, 0.0,
                      (double)b->n_values * 2.0 * (value_kind ? 8.0 : 4.0) +
                          (double)n_k * (double)b->nnz * 2.0 * 8.0);
-  return aosb::launch_check(err, cap, "bloch_strips_kernel");
+  return aosb::launch_check(err, cap, "bloch sums");
 }
 
 void aosb_bloch_destroy(aosb_bloch_t* b) {
@@ -586,6 +737,7 @@ void aosb_bloch_destroy(aosb_bloch_t* b) {
   cudaFree(b->d_member_off);
   cudaFree(b->d_member_shift);
   cudaFree(b->d_strips);
+  cudaFree(b->d_others);
   delete b;
 }
 
